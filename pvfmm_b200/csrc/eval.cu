@@ -39,6 +39,8 @@
 #include <cstring>
 #include <functional>
 
+#include <cuda_fp16.h>
+
 #include "fmm_context.cuh"
 
 namespace pvfmm_b200 {
@@ -848,6 +850,61 @@ __global__ void __launch_bounds__(kNT) surface_check_kernel(
 // size is a compile-time constant.  A block handles G grids (child x
 // component) of one parent.
 // ---------------------------------------------------------------------------
+
+// ---------------------------------------------------------------------------
+// Split-FP16 spectra of the mixed form's Hadamards.  A value v of parent q is
+// stored as hi = fp16(v 2^-E), lo = fp16(v 2^-E - hi) (22 bits and lo's sign,
+// as a TF32 hi/lo pair), with one exponent E per parent such that no value of
+// its spectra exceeds 2^15.  Values down to 2^-18 of that bound keep all 22
+// bits; below that the error stays at 2^-25, 2^-40 of the bound.
+// ---------------------------------------------------------------------------
+// (re, im) as two packed halves: their hi parts and their lo parts.
+__device__ __forceinline__ void half_split(float re, float im, unsigned& hi, unsigned& lo) {
+  const __half2 h = __floats2half2_rn(re, im);
+  const float2 hf = __half22float2(h);
+  const __half2 l = __floats2half2_rn(re - hf.x, im - hf.y);
+  memcpy(&hi, &h, 4);
+  memcpy(&lo, &l, 4);
+}
+// Row of frequency f, parent q (n_q parents): frequency-major, so that the
+// rows which the blocks of one frequency gather lie together (m = 8: 64 bytes
+// each, 1 MB for 16k parents).
+__device__ __forceinline__ long split_row(int f, long q, long n_q) { return (long)f * n_q + q; }
+// Word of element e's hi part in its row (its lo part is 2 words on): elements
+// 2k and 2k+1 share one 16-byte piece (hi, hi, lo, lo), the hi and lo A
+// fragments of one lane.
+__device__ __forceinline__ int split_word(int e) { return (e >> 1) * 4 + (e & 1); }
+
+// Exponents of the parents' spectra: |spectrum value| <= sum |density| of its
+// child, so E = (exponent of the largest such sum over the 8 children) - 15;
+// qscale = 2^E, qinv = 2^-E.  One block of 8 warps per parent, one child per
+// warp; `len` values per child.  A sum that is zero or not finite leaves E = 0.
+__global__ void __launch_bounds__(256) vsrc_scale_kernel(const int* __restrict__ vsrc, const int* __restrict__ child0,
+                                                         const double* __restrict__ ue, int len,
+                                                         float* __restrict__ qscale, double* __restrict__ qinv) {
+  __shared__ double part[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double* row = ue + (long)(child0[vsrc[blockIdx.x]] + warp) * len;
+  double sum = 0;
+  for (int i = lane; i < len; i += 32) sum += fabs(row[i]);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+  if (lane == 0) part[warp] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double top = 0;
+    bool finite = true;
+    for (int c = 0; c < 8; ++c) {
+      finite = finite && isfinite(part[c]);
+      top = fmax(top, part[c]);
+    }
+    int e = 15;
+    if (finite && top > 0) frexp(top, &e);
+    qscale[blockIdx.x] = (float)ldexp(1.0, e - 15);
+    qinv[blockIdx.x] = ldexp(1.0, 15 - e);
+  }
+}
+
 template <class Real, int M>
 struct FftSizes {
   static constexpr int N1 = 2 * M, NH = M + 1, M3 = M * M * M, N3H = N1 * N1 * NH;
@@ -868,14 +925,16 @@ struct FftSizes {
 // (twiddle index (k * x) mod N1 known at compile time, read as a broadcast).
 // Output layout: FP64 with ke == 1 writes the spectra piece-major,
 // spec[f][child][q] (16 bytes per child), so that the scalar Hadamard's
-// gathers over Morton-adjacent parents coalesce; otherwise rows
-// spec[q][f][child*ke+comp] (the tensor-core Hadamard reads a 64-byte FP32
-// row with four lanes).
+// gathers over Morton-adjacent parents coalesce; FP32 with `qscale` (the
+// split-FP16 Hadamards) writes each value times 2^-E of its parent
+// (qscale[q] = 2^E) as FP16 hi + lo in the order of split_word; otherwise
+// rows spec[q][f][child*ke+comp].
 template <class Real, int M>
 __global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups, const int* __restrict__ vsrc,
                                                       const int* __restrict__ child0, const double* __restrict__ ue,
                                                       const int* __restrict__ fft_map, int ns, long n_q, int kz0,
-                                                      int nkz, Cplx<Real>* __restrict__ spec) {
+                                                      int nkz, const double* __restrict__ qinv,
+                                                      Cplx<Real>* __restrict__ spec) {
   using F = FftSizes<Real, M>;
   constexpr int N1 = F::N1, NH = F::NH, M3 = F::M3, N3H = F::N3H, A2S = F::A2S;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -891,6 +950,7 @@ __global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups,
   const int P = vsrc[q];
   const int c0 = child0[P];
   const int dim = ns * ke;
+  const double ascale = qinv ? qinv[q] : 1.0;
   for (int j = threadIdx.x; j < N1; j += blockDim.x) {
     double sn, cs;
     sincospi(-2.0 * j / N1, &sn, &cs);
@@ -904,7 +964,7 @@ __global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups,
     const int gg = gb + gi, c = gg / ke, comp = gg % ke;
     const int idx = fft_map[k];  // x + N1*y + N1*N1*z, all < M
     const int x = idx % N1, y = (idx / N1) % N1, z = idx / (N1 * N1);
-    g[gi * M3 + x + M * (y + M * z)] = (Real)ue[(long)(c0 + c) * dim + k * ke + comp];
+    g[gi * M3 + x + M * (y + M * z)] = (Real)(ue[(long)(c0 + c) * dim + k * ke + comp] * ascale);
   }
   __syncthreads();
   // x -> kx (real input): line = (gi, z, y)
@@ -968,8 +1028,17 @@ __global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups,
         im += v[z].re * twi[w] + v[z].im * twr[w];
       }
       const int f = l + N1 * NH * (kz - kz0);
-      if (sizeof(Real) == 8 && ke == 1) spec[((long)f * 8 + gb + gi) * n_q + q] = {re, im};
-      else out[(long)f * ngrid + gb + gi] = {re, im};
+      if (sizeof(Real) == 8 && ke == 1) {
+        spec[((long)f * 8 + gb + gi) * n_q + q] = {re, im};
+      } else if (sizeof(Real) == 4 && qinv) {
+        unsigned hi, lo;
+        half_split((float)re, (float)im, hi, lo);
+        unsigned* w = reinterpret_cast<unsigned*>(spec) + split_row(f, q, n_q) * (2 * ngrid) + split_word(gb + gi);
+        w[0] = hi;
+        w[2] = lo;
+      } else {
+        out[(long)f * ngrid + gb + gi] = {re, im};
+      }
     }
   }
 }
@@ -1311,240 +1380,229 @@ __global__ void __launch_bounds__(128, 4) hadamard_rd_kernel(int n3h, long n_vtr
 }
 
 // ---------------------------------------------------------------------------
-// Hadamard products of the mixed form (ke = 1) on the tensor cores:
-// mma.sync m16n8k8 TF32 with FP32 accumulation, each product split into
-// three (a_hi b_hi + a_hi b_lo + a_lo b_hi, hi = the value rounded to TF32,
-// lo = the remainder rounded to TF32), which carries the products to ~2^-22
-// relative (an emulation of the whole FMM with this split changes the result
-// by ~1e-8 relative).
+// Hadamard products of the mixed form (scalar expansions here, 3-component
+// ones below) on the tensor cores: mma.sync m16n8k16 on split-FP16 spectra and operators with FP32 accumulation, three products
+// per value (a_lo b_hi + a_hi b_lo + a_hi b_hi), which carries the products to
+// ~2^-22 relative.
 //
 // Per frequency f the product is a real GEMM over parent rows:
-//   OUT[P][(j1, re|im)] += sum_o sum_(j2, re|im) IN[Q_o(P)][(j2, re|im)] * B_o[(j2, re|im)][(j1, re|im)]
-// with B_o the real form of the complex 8x8 block M[f][o].  A warp owns MT
-// tiles of 16 target parents.  The A fragments come straight from the input
-// spectrum rows in L2: lane (g, t) loads the 16-byte piece t (children 2t and
-// 2t+1, re and im) of rows g and g+8 (four lanes read one 64-byte row), which
-// is exactly its fragment once the K order is chosen as k-step s, column
-// c -> float 4t + 2s (+1 for c = t + 4).  The B fragments of every (f, o, lane) are precomputed on the
-// host in that order, hi and lo, and staged per block in shared memory.
+//   OUT[P][(e_out, re|im)] += sum_o sum_(e, re|im) IN[Q_o(P)][(e, re|im)] * B_o[(e, re|im)][(e_out, re|im)]
+// with elements e = child * ke + component and B_o the real form of the
+// complex block M[f][o].  A warp owns 16-row tiles of target parents.  The A
+// fragments come straight from the input rows in L2: lane (g, t) loads the
+// 16-byte piece t of each 8 elements (elements 2t and 2t+1: hi re|im of both,
+// then lo) of rows g and g+8 (four lanes read 64 contiguous bytes), which is
+// its hi and lo fragment when the K order of the k-step is chosen as columns
+// 2t, 2t+1 -> element 2t (re, im), columns 2t+8, 2t+9 -> element 2t+1.  No
+// conversion is left in the loop.  The products of one offset accumulate in a
+// fresh fragment that joins the running sum with a rounded FP32 fma, times the
+// source parent's 2^E: the tensor cores' own FP32 accumulation is not
+// round-to-nearest and, carried over all 26 offsets, left a bias of ~2e-6 in
+// the far-field potential.
+// Why FP16: the same 11-bit halves as a TF32 hi/lo pair at twice the MMA rate
+// (measured 554 against 276 TFLOP/s for mma.sync), with half the operator
+// bytes, and the split is done once per spectrum value by the forward DFT
+// instead of at each of its up to 26 uses (24 conversions and subtractions
+// per 16 rows and offset).  Measured against that TF32 form: 4M clustered
+// points (m = 8, 16,037 parents) 10.8 -> 7.05 ms, 2M surface points 13.1 ->
+// 7.5 ms, 1M Stokes points (m = 6) 9.5 -> 6.1 ms; outputs 3e-9 to 9e-7 apart.
+// What bounds the scalar kernel now is the L1 data path (72% of its rate: 12
+// wavefronts for the two gathers of a tile and offset, 8 for the operator
+// fragments, 4 for scales and indices, against 13 cycles of MMA), with 59% of
+// the gathered sectors hit in L1; so the kernel keeps its shared memory small:
+// operator fragments 27 KB per block, 3 blocks per SM (4 blocks, with a
+// smaller L1, took 9.0 ms; two tiles per warp 7.7 ms).  Each warp prefetches
+// the index table of its next tile by itself (a block-wide table behind a
+// barrier: 7.4 ms, surface 8.6 ms).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void mma_tf32_16x8x8(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+// d = a b (zero accumulator) and d += a b
+__device__ __forceinline__ void mma_f16_zero(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
+                                             unsigned b0, unsigned b1) {
   asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%10,%10,%10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void mma_f16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
+                                        unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// The three products of one k-step: rows g (x) and g+8 (y), b = (hi, hi, lo, lo).
+__device__ __forceinline__ void mma_split(float (&d)[4], const uint4& x, const uint4& y, const uint4& b) {
+  mma_f16_zero(d, x.z, y.z, x.w, y.w, b.x, b.y);
+  mma_f16(d, x.x, y.x, x.y, y.y, b.z, b.w);
+  mma_f16(d, x.x, y.x, x.y, y.y, b.x, b.y);
 }
 
-// hi = x rounded to TF32 (cvt.rna), lo = (x - hi) rounded to TF32: hi + lo
-// carries x to ~2^-23 relative.  (Passing unrounded FP32 values leaves the
-// conversion to the MMA's truncation, up to 2^-20 relative per product,
-// which showed as ~1e-6 in the FMM result.)
-__device__ __forceinline__ void tf32_split(float x, unsigned& hi, unsigned& lo) {
-  unsigned h, l;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-  const float r = x - __uint_as_float(h);
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(r));
-  hi = h;
-  lo = l;
-}
-
-constexpr int kTcWarps = 8;  // warps per block of the tensor-core Hadamard
+#ifndef PVFMM_TC_WARPS
+#define PVFMM_TC_WARPS 8
+#endif
+constexpr int kTcWarps = PVFMM_TC_WARPS;  // warps per block of the scalar tensor-core Hadamard
 #ifndef PVFMM_TC_MIN_BLOCKS
-#define PVFMM_TC_MIN_BLOCKS 2
+#define PVFMM_TC_MIN_BLOCKS 3
 #endif
 #ifndef PVFMM_TC_CHUNKS
-#define PVFMM_TC_CHUNKS 8  // target-parent chunks per block (operator fragments staged once)
+#define PVFMM_TC_CHUNKS 16  // tiles per warp (operator fragments staged once)
 #endif
 
-template <int MT>
-__global__ void __launch_bounds__(32 * kTcWarps, PVFMM_TC_MIN_BLOCKS) hadamard_tc_kernel(int n3h, long n_vtrg, long vt_stride, long n_vsrc,
-                                                                       int chunks,
-                                                                       const int* __restrict__ vtab,
-                                                                       const unsigned* __restrict__ vmask,
-                                                                       const float4* __restrict__ spec_in,
-                                                                       const float4* __restrict__ bfrag,
-                                                                       float2* __restrict__ spec_out) {
-  extern __shared__ float4 Bs[];  // [26 offsets][4 blocks (s, nt)][32 lanes]: (b0 hi, b1 hi, b0 lo, b1 lo)
-  constexpr int NP = kTcWarps * 16 * MT;  // target parents of a chunk
-  int* qs = reinterpret_cast<int*>(Bs + 26 * 4 * 32);  // [26][NP] source parent of each (offset, parent)
-  unsigned* ms = reinterpret_cast<unsigned*>(qs + 26 * NP);  // [NP] occupied-offset pattern of each parent
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
+}
+
+#ifndef PVFMM_TC_STAGES
+#define PVFMM_TC_STAGES 3
+#endif
+constexpr int kTcEnt = 26 * 16 + 16;  // words of a tile's table: source parents [26][16], patterns [16]
+
+__global__ void __launch_bounds__(32 * kTcWarps, PVFMM_TC_MIN_BLOCKS)
+    hadamard_tc_kernel(int n3h, long n_vtrg, long vt_stride, long n_vsrc, int chunks, const int* __restrict__ vtab,
+                       const unsigned* __restrict__ vmask, const uint4* __restrict__ spec_in,
+                       const float* __restrict__ qscale, const uint4* __restrict__ bfrag,
+                       const float* __restrict__ fscale, float2* __restrict__ spec_out) {
+  extern __shared__ uint4 Bs[];  // [26 offsets][2 n-tiles][32 lanes], then two tables per warp
   const int f = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  {
-    const float4* src = bfrag + (long)f * 26 * 4 * 32;
-    for (int i = threadIdx.x; i < 26 * 4 * 32; i += 32 * kTcWarps) Bs[i] = __ldg(src + i);
-  }
-  // the block's operator fragments stay staged over `chunks` chunks of NP
-  // target parents (the condition below is uniform across the block)
-  for (int c = 0; c < chunks; ++c) {
-    const long pb = ((long)blockIdx.x * chunks + c) * NP;
-    if (pb >= n_vtrg) break;
-    if (c > 0) __syncthreads();  // every warp is done with the previous chunk's qs
-    for (int i = threadIdx.x; i < 26 * NP; i += 32 * kTcWarps) {
-      const int o = i / NP;
-      const long p = pb + i % NP;
-      qs[i] = p < n_vtrg ? __ldg(vtab + (long)o * vt_stride + p) : -1;
+  int* ent = reinterpret_cast<int*>(Bs + 26 * 2 * 32) + warp * 2 * kTcEnt;
+  // table of the warp's tile c into buffer c % 2 (rows past the end repeat the
+  // last parent; their sums are not stored)
+  auto tile_p0 = [&](int c) { return ((long)(blockIdx.x * chunks + c) * kTcWarps + warp) * 16; };
+  auto fetch = [&](int c) {
+    const long p0 = tile_p0(c);
+    if (c < chunks && p0 < n_vtrg) {
+      const long p = min(p0 + (lane & 15), n_vtrg - 1);
+      int* dst = ent + (c & 1) * kTcEnt + lane;
+      const int* src = vtab + (long)(lane >> 4) * vt_stride + p;
+#pragma unroll
+      for (int o = 0; o < 26; o += 2) cp_async4(dst + o * 16, src + (long)o * vt_stride);
+      if (lane < 16) cp_async4(dst + 26 * 16, vmask + p);
     }
-    for (int i = threadIdx.x; i < NP; i += 32 * kTcWarps) ms[i] = pb + i < n_vtrg ? __ldg(vmask + pb + i) : 0u;
-    __syncthreads();
-    const int w0 = warp * 16 * MT;  // first parent of the warp within the chunk
-    const long p0 = pb + w0;
-    const float4* in_f = spec_in + (long)f * 4 + t;  // row q: in_f[q * n3h * 4]
-    float acc[MT][2][4];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[mt][nt][i] = 0.f;
-    float4 xa[MT][2], xb[MT][2], xc[MT][2];
-    // offsets without a source parent for any of the warp's parents are
+    cp_async_commit();
+  };
+  fetch(0);
+  {
+    const uint4* src = bfrag + (long)f * 26 * 2 * 32;
+    for (int i = threadIdx.x; i < 26 * 2 * 32; i += 32 * kTcWarps) Bs[i] = __ldg(src + i);
+  }
+  const float fs = fscale[f];
+  const uint4* in_f = spec_in + split_row(f, 0, n_vsrc) * 4 + t;  // row q: in_f[q * 4]
+  __syncthreads();  // the operator fragments are staged
+  for (int c = 0; c < chunks; ++c) {
+    const long p0 = tile_p0(c);
+    if (p0 >= n_vtrg) break;
+    cp_async_wait<0>();
+    __syncwarp();  // the tile's table has landed, and the other buffer is no longer read
+    fetch(c + 1);
+    const int* qs = ent + (c & 1) * kTcEnt + g;
+    // offsets without a source parent for any of the tile's parents are
     // neither loaded nor multiplied (their products are zero); the targets
     // are ordered by occupied-offset pattern, so such offsets are common
-    unsigned live = 0;
-    for (int k = lane; k < 16 * MT; k += 32) live |= ms[w0 + k];
-    live = __reduce_or_sync(0xffffffffu, live);
-    auto load = [&](int o, float4 (&x)[MT][2]) {
+    unsigned rem = __reduce_or_sync(0xffffffffu, (unsigned)ent[(c & 1) * kTcEnt + 26 * 16 + (lane & 15)]);
+    float acc[2][4];
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+    for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int q = qs[o * NP + w0 + mt * 16 + g + 8 * h];
-          x[mt][h] = q >= 0 ? __ldg(in_f + (long)q * n3h * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+      for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
+    struct Rows {
+      uint4 x[2];
+      float s[2];
     };
-    auto compute = [&](int o, const float4 (&x)[MT][2]) {
-      float4 bq[4];
+    auto load = [&](int o, Rows& r) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) bq[i] = Bs[(o * 4 + i) * 32 + lane];  // consecutive lanes: conflict-free
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        unsigned ah[2][4], al[2][4];
-        tf32_split(x[mt][0].x, ah[0][0], al[0][0]);
-        tf32_split(x[mt][1].x, ah[0][1], al[0][1]);
-        tf32_split(x[mt][0].y, ah[0][2], al[0][2]);
-        tf32_split(x[mt][1].y, ah[0][3], al[0][3]);
-        tf32_split(x[mt][0].z, ah[1][0], al[1][0]);
-        tf32_split(x[mt][1].z, ah[1][1], al[1][1]);
-        tf32_split(x[mt][0].w, ah[1][2], al[1][2]);
-        tf32_split(x[mt][1].w, ah[1][3], al[1][3]);
-        // this offset's products accumulate in a fresh fragment and join the
-        // running sum with rounded FP32 adds: the tensor cores' own FP32
-        // accumulation is not round-to-nearest and, carried over all 26
-        // offsets, left a bias of ~2e-6 in the far-field potential
-        float d[2][4];
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) d[nt][i] = 0.f;
-#pragma unroll
-        for (int s = 0; s < 2; ++s)
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            const float4 b = bq[s * 2 + nt];
-            const unsigned bh0 = __float_as_uint(b.x), bh1 = __float_as_uint(b.y);
-            const unsigned bl0 = __float_as_uint(b.z), bl1 = __float_as_uint(b.w);
-            mma_tf32_16x8x8(d[nt], al[s], bh0, bh1);
-            mma_tf32_16x8x8(d[nt], ah[s], bl0, bl1);
-            mma_tf32_16x8x8(d[nt], ah[s], bh0, bh1);
-          }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[mt][nt][i] += d[nt][i];
+      for (int h = 0; h < 2; ++h) {
+        const int q = qs[o * 16 + 8 * h];
+        r.x[h] = q >= 0 ? __ldg(in_f + (long)q * 4) : make_uint4(0u, 0u, 0u, 0u);
+        r.s[h] = q >= 0 ? __ldg(qscale + q) : 0.f;
       }
     };
-    // The warp's occupied offsets in increasing order, one set bit at a
-    // time; three register sets in turn: the gathers of the next two offsets
-    // are in flight while one offset is multiplied.
-    unsigned rem = live;
-    const int nlive = __popc(live);
-    auto take = [&]() {
-      const int o = __ffs(rem) - 1;
-      rem &= rem - 1;
-      return o;
+    auto compute = [&](int o, const Rows& r) {
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        float d[4];
+        mma_split(d, r.x[0], r.x[1], Bs[(o * 2 + nt) * 32 + lane]);  // consecutive lanes: conflict-free
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[nt][i] = fmaf(d[i], r.s[i >> 1], acc[nt][i]);
+      }
     };
-    int oa = 0, ob = 0, oc = 0;
-    if (nlive > 0) {
-      oa = take();
-      load(oa, xa);
-    }
-    if (nlive > 1) {
-      ob = take();
-      load(ob, xb);
-    }
+    // The tile's occupied offsets in increasing order, one set bit at a time,
+    // kStages register sets in turn: the gathers of the next offsets are in
+    // flight while one is multiplied.
+    constexpr int kStages = PVFMM_TC_STAGES;
+    const int nlive = __popc(rem);
+    Rows r[kStages];
+    int o[kStages];
+#pragma unroll
+    for (int k = 0; k < kStages - 1; ++k)
+      if (k < nlive) {
+        o[k] = __ffs(rem) - 1;
+        rem &= rem - 1;
+        load(o[k], r[k]);
+      }
 #pragma unroll 1
-    for (int i = 0; i < nlive; i += 3) {
-      if (i + 2 < nlive) {
-        oc = take();
-        load(oc, xc);
+    for (int i = 0; i < nlive; i += kStages) {
+#pragma unroll
+      for (int k = 0; k < kStages; ++k) {
+        constexpr int kAhead = kStages - 1;
+        const int n = (k + kAhead) % kStages;
+        if (i + k + kAhead < nlive) {
+          o[n] = __ffs(rem) - 1;
+          rem &= rem - 1;
+          load(o[n], r[n]);
+        }
+        if (k == 0 || i + k < nlive) compute(o[k], r[k]);
       }
-      compute(oa, xa);
-      if (i + 3 < nlive) {
-        oa = take();
-        load(oa, xa);
-      }
-      if (i + 1 < nlive) compute(ob, xb);
-      if (i + 4 < nlive) {
-        ob = take();
-        load(ob, xb);
-      }
-      if (i + 2 < nlive) compute(oc, xc);
     }
     // C fragment: (row g, cols 2t, 2t+1) and (row g+8, same cols); column
     // n = nt*8 + 2t (+1) is child j1 = 4nt + t, re (im).
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int h = 0; h < 2; ++h) {
+      const long p = p0 + g + 8 * h;
+      if (p >= n_vtrg) continue;
+      float2* out = spec_out + (p * n3h + f) * 8;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const long p = p0 + mt * 16 + g + 8 * h;
-        if (p >= n_vtrg) continue;
-        float2* out = spec_out + (p * n3h + f) * 8;
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) out[4 * nt + t] = make_float2(acc[mt][nt][2 * h], acc[mt][nt][2 * h + 1]);
-      }
+      for (int nt = 0; nt < 2; ++nt) out[4 * nt + t] = make_float2(acc[nt][2 * h] * fs, acc[nt][2 * h + 1] * fs);
+    }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Hadamard products of the mixed form for 3-component expansions (Stokes
-// velocity, pressure and velocity gradient, Biot-Savart) on the tensor cores,
-// with the same TF32 3-term split as hadamard_tc_kernel.  Per frequency f and
-// group z of KOC output components:
-//   OUT[P][(j1, c, re|im)] += sum_o sum_(j2, i, re|im) IN[Q_o(P)][(j2, i, re|im)] B_o[..][(j1, c, re|im)]
-// a real GEMM with K = 48 (8 children x 3 components x re|im, 6 k-steps) and
-// N = 16 KOC (2 KOC n-tiles), B_o the real form of the complex block
-// M[f][o][(j1, c)][(j2, i)].  A warp owns 16 target parents (rows); lane
-// (g, t) loads the 16-byte pieces u = 0..2 at float 16u + 4t of the 48-float
-// input rows g and g+8, which are its A fragments for k-steps 2u and 2u+1
-// when the K order is chosen as k-step 2u+v, column c -> float
-// 16u + 4(c % 4) + 2v + c / 4.  The B fragments of an offset (18 KB for
-// KOC = 3) are too many to stage for all 26 offsets, so the block streams
-// them, PVFMM_TC3_OPB offsets at a time, into a double buffer in shared
-// memory (cp.async, one barrier per group; two offsets per group measured
-// 3% faster than one at 2M Stokes points), shared by its 8 warps; offsets that no parent of
-// the block has are skipped, those that no parent of a warp has are skipped
-// by that warp.  Each pair of k-steps accumulates in a fresh fragment that
-// joins the running sum with a rounded FP32 add (see hadamard_tc_kernel).
+// The same for 3-component expansions (Stokes velocity, pressure and velocity
+// gradient, Biot-Savart), per group z of KOC output components: K = 48 (24
+// elements, 3 k-steps of 8) and N = 16 KOC (2 KOC n-tiles).  A warp owns 16
+// target parents; lane (g, t) loads the 16-byte pieces 4u + t, u = 0..2, of
+// the 192-byte rows g and g+8.  The B fragments of an offset (9 KB for KOC =
+// 3) are too many to stage for all 26 offsets, so the block streams them,
+// PVFMM_TC3_OPB offsets at a time, into a double buffer in shared memory
+// (cp.async, one barrier per group), shared by its 8 warps; offsets that no
+// parent of the block has are skipped, those that no parent of a warp has are
+// skipped by that warp.  Each k-step accumulates in a fresh fragment.
 // ---------------------------------------------------------------------------
 constexpr int kTc3Warps = 8;
 #ifndef PVFMM_TC3_OPB
-#define PVFMM_TC3_OPB 2  // offsets whose B fragments are staged per barrier
+#define PVFMM_TC3_OPB 4  // offsets whose B fragments are staged per barrier (1M Stokes points: 2 6.22, 4 6.14 ms)
 #endif
 constexpr int kTc3Opb = PVFMM_TC3_OPB;
+#ifndef PVFMM_TC3_MIN_BLOCKS
+#define PVFMM_TC3_MIN_BLOCKS 2
+#endif
 
 template <int KOC>
-__global__ void __launch_bounds__(32 * kTc3Warps, 2)
-    hadamard_tc3_kernel(int n3h, long n_vtrg, long vt_stride, int ko, const int* __restrict__ vtab,
-                        const unsigned* __restrict__ vmask, const float4* __restrict__ spec_in,
-                        const float4* __restrict__ bfrag, float2* __restrict__ spec_out) {
+__global__ void __launch_bounds__(32 * kTc3Warps, PVFMM_TC3_MIN_BLOCKS)
+    hadamard_tc3_kernel(int n3h, long n_vtrg, long vt_stride, long n_vsrc, int ko, const int* __restrict__ vtab,
+                        const unsigned* __restrict__ vmask, const uint4* __restrict__ spec_in,
+                        const float* __restrict__ qscale, const uint4* __restrict__ bfrag,
+                        const float* __restrict__ fscale, float2* __restrict__ spec_out) {
   constexpr int NNT = 2 * KOC;        // n-tiles of the group
-  constexpr int NB = 6 * NNT;         // (k-step, n-tile) fragment blocks per offset
+  constexpr int NB = 3 * NNT;         // (k-step, n-tile) fragment blocks per offset
   constexpr int NP = kTc3Warps * 16;  // target parents of the block
   constexpr int OPB = kTc3Opb;
-  extern __shared__ float4 Bs[];      // [2][OPB][NB][32 lanes]: (b0 hi, b1 hi, b0 lo, b1 lo)
+  extern __shared__ uint4 Bs[];       // [2][OPB][NB][32 lanes]: (b0 hi, b1 hi, b0 lo, b1 lo)
   int* qs = reinterpret_cast<int*>(Bs + 2 * OPB * NB * 32);  // [26][NP] source parent of each (offset, parent)
   unsigned* wl = reinterpret_cast<unsigned*>(qs + 26 * NP);  // [kTc3Warps] occupied offsets of each warp
   const int f = blockIdx.y, z = blockIdx.z, ngroups = gridDim.z;
@@ -1567,7 +1625,8 @@ __global__ void __launch_bounds__(32 * kTc3Warps, 2)
 #pragma unroll
   for (int w = 0; w < kTc3Warps; ++w) blive |= wl[w];
   const unsigned wlive = wl[warp];
-  const float4* bsrc = bfrag + ((long)f * 26 * ngroups + z) * NB * 32;  // + o * ngroups * NB * 32
+  const float fs = fscale[f];
+  const uint4* bsrc = bfrag + ((long)f * 26 * ngroups + z) * NB * 32;  // + o * ngroups * NB * 32
   // the next (up to) OPB block-live offsets of srem into buffer buf
   unsigned srem = blive;
   auto stage_group = [&](int buf) {
@@ -1576,19 +1635,25 @@ __global__ void __launch_bounds__(32 * kTc3Warps, 2)
       if (!srem) break;
       const int o = __ffs(srem) - 1;
       srem &= srem - 1;
-      const float4* src = bsrc + (long)o * ngroups * NB * 32;
-      float4* dst = Bs + (buf * OPB + j) * NB * 32;
+      const uint4* src = bsrc + (long)o * ngroups * NB * 32;
+      uint4* dst = Bs + (buf * OPB + j) * NB * 32;
       for (int i = threadIdx.x; i < NB * 32; i += 32 * kTc3Warps) cp_async16(dst + i, src + i, 16);
     }
   };
   const int w0 = warp * 16;
-  auto load = [&](int o, float4 (&x)[3][2]) {
+  const uint4* in_f = spec_in + split_row(f, 0, n_vsrc) * 12 + t;
+  struct Rows {
+    uint4 x[3][2];
+    float s[2];
+  };
+  auto load = [&](int o, Rows& r) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int q = qs[o * NP + w0 + g + 8 * h];
-      const float4* row = spec_in + ((long)(q < 0 ? 0 : q) * n3h + f) * 12 + t;
+      const uint4* row = in_f + (long)(q < 0 ? 0 : q) * 12;
 #pragma unroll
-      for (int u = 0; u < 3; ++u) x[u][h] = q >= 0 ? __ldg(row + 4 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int u = 0; u < 3; ++u) r.x[u][h] = q >= 0 ? __ldg(row + 4 * u) : make_uint4(0u, 0u, 0u, 0u);
+      r.s[h] = q >= 0 ? __ldg(qscale + q) : 0.f;
     }
   };
   float acc[NNT][4];
@@ -1596,7 +1661,7 @@ __global__ void __launch_bounds__(32 * kTc3Warps, 2)
   for (int nt = 0; nt < NNT; ++nt)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
-  float4 xn[3][2];
+  Rows xc, xn;
   unsigned rem = blive;
   int oc = rem ? __ffs(rem) - 1 : 0;
   if (rem) {
@@ -1616,37 +1681,17 @@ __global__ void __launch_bounds__(32 * kTc3Warps, 2)
       cp_async_commit();
     }
     if (wlive >> oc & 1u) {
-      unsigned ah[6][4], al[6][4];
-#pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        tf32_split(xn[u][0].x, ah[2 * u][0], al[2 * u][0]);
-        tf32_split(xn[u][1].x, ah[2 * u][1], al[2 * u][1]);
-        tf32_split(xn[u][0].y, ah[2 * u][2], al[2 * u][2]);
-        tf32_split(xn[u][1].y, ah[2 * u][3], al[2 * u][3]);
-        tf32_split(xn[u][0].z, ah[2 * u + 1][0], al[2 * u + 1][0]);
-        tf32_split(xn[u][1].z, ah[2 * u + 1][1], al[2 * u + 1][1]);
-        tf32_split(xn[u][0].w, ah[2 * u + 1][2], al[2 * u + 1][2]);
-        tf32_split(xn[u][1].w, ah[2 * u + 1][3], al[2 * u + 1][3]);
-      }
+      xc = xn;
       if (on >= 0 && (wlive >> on & 1u)) load(on, xn);  // the next offset's rows, in flight meanwhile
-      const float4* bq = Bs + ((grp & 1) * OPB + slot) * NB * 32 + lane;
+      const uint4* bq = Bs + ((grp & 1) * OPB + slot) * NB * 32 + lane;
 #pragma unroll
       for (int nt = 0; nt < NNT; ++nt)
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
-          float d[4] = {0.f, 0.f, 0.f, 0.f};
+          float d[4];
+          mma_split(d, xc.x[u][0], xc.x[u][1], bq[(u * NNT + nt) * 32]);
 #pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            const int sk = 2 * u + v;
-            const float4 b = bq[(sk * NNT + nt) * 32];
-            const unsigned bh0 = __float_as_uint(b.x), bh1 = __float_as_uint(b.y);
-            const unsigned bl0 = __float_as_uint(b.z), bl1 = __float_as_uint(b.w);
-            mma_tf32_16x8x8(d, al[sk], bh0, bh1);
-            mma_tf32_16x8x8(d, ah[sk], bl0, bl1);
-            mma_tf32_16x8x8(d, ah[sk], bh0, bh1);
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[nt][i] += d[i];
+          for (int i = 0; i < 4; ++i) acc[nt][i] = fmaf(d[i], xc.s[i >> 1], acc[nt][i]);
         }
     } else if (on >= 0 && (wlive >> on & 1u)) {
       load(on, xn);
@@ -1665,7 +1710,7 @@ __global__ void __launch_bounds__(32 * kTc3Warps, 2)
 #pragma unroll
     for (int nt = 0; nt < NNT; ++nt) {
       const int e = 4 * nt + t;
-      out[(e / KOC) * ko + e % KOC] = make_float2(acc[nt][2 * h], acc[nt][2 * h + 1]);
+      out[(e / KOC) * ko + e % KOC] = make_float2(acc[nt][2 * h] * fs, acc[nt][2 * h + 1] * fs);
     }
   }
 }
@@ -1674,16 +1719,17 @@ template <int KOC>
 void launch_hadamard_tc3(Context& ctx, int n3h, long f_base, int ko, const Cplx<float>* sin_, Cplx<float>* sout,
                          long p0, long np) {
   DevTree& T = ctx.tree;
-  constexpr int NB = 12 * KOC, NP = kTc3Warps * 16;
+  constexpr int NB = 6 * KOC, NP = kTc3Warps * 16;
   const int ngroups = ko / KOC;
-  const size_t sm = (size_t)2 * kTc3Opb * NB * 32 * sizeof(float4) + (size_t)26 * NP * sizeof(int) +
+  const size_t sm = (size_t)2 * kTc3Opb * NB * 32 * sizeof(uint4) + (size_t)26 * NP * sizeof(int) +
                     kTc3Warps * sizeof(int);
   PVFMM_CUDA_CHECK(cudaFuncSetAttribute(hadamard_tc3_kernel<KOC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   dim3 grid(ceil_div(np, (long)NP), n3h, ngroups);
   ++ctx.n_launch;
   hadamard_tc3_kernel<KOC><<<grid, 32 * kTc3Warps, sm, ctx.stream>>>(
-      n3h, np, T.n_vtrg, ko, T.vtab.get<int>() + p0, T.vmask.get<unsigned>() + p0,
-      reinterpret_cast<const float4*>(sin_), ctx.dops.vop_frag.get<float4>() + f_base * 26 * ngroups * NB * 32,
+      n3h, np, T.n_vtrg, T.n_vsrc, ko, T.vtab.get<int>() + p0, T.vmask.get<unsigned>() + p0,
+      reinterpret_cast<const uint4*>(sin_), ctx.qscale.get<float>(),
+      ctx.dops.vop_frag.get<uint4>() + f_base * 26 * ngroups * NB * 32, ctx.dops.vop_fscale.get<float>() + f_base,
       reinterpret_cast<float2*>(sout));
 }
 
@@ -1956,16 +2002,16 @@ void launch_hadamard_dmma3(Context& ctx, int n3h, long f_base, int ko, const Cpl
 void launch_hadamard_tc(Context& ctx, int n3h, long f_base, const Cplx<float>* sin_, Cplx<float>* sout, long p0,
                         long np) {
   DevTree& T = ctx.tree;
-  constexpr int MT = 2;
-  const size_t sm = (size_t)26 * 4 * 32 * sizeof(float4) + (size_t)27 * kTcWarps * 16 * MT * sizeof(int);
-  PVFMM_CUDA_CHECK(cudaFuncSetAttribute(hadamard_tc_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  const size_t sm = (size_t)26 * 2 * 32 * sizeof(uint4) + (size_t)kTcWarps * 2 * kTcEnt * sizeof(int);
+  PVFMM_CUDA_CHECK(cudaFuncSetAttribute(hadamard_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int chunks = PVFMM_TC_CHUNKS;
-  dim3 grid(ceil_div(np, (long)16 * MT * kTcWarps * chunks), n3h);
+  dim3 grid(ceil_div(np, (long)16 * kTcWarps * chunks), n3h);
   ++ctx.n_launch;
-  hadamard_tc_kernel<MT><<<grid, 32 * kTcWarps, sm, ctx.stream>>>(
+  hadamard_tc_kernel<<<grid, 32 * kTcWarps, sm, ctx.stream>>>(
       n3h, np, T.n_vtrg, T.n_vsrc, chunks, T.vtab.get<int>() + p0, T.vmask.get<unsigned>() + p0,
-      reinterpret_cast<const float4*>(sin_),
-      ctx.dops.vop_frag.get<float4>() + f_base * 26 * 4 * 32, reinterpret_cast<float2*>(sout));
+      reinterpret_cast<const uint4*>(sin_), ctx.qscale.get<float>(),
+      ctx.dops.vop_frag.get<uint4>() + f_base * 26 * 2 * 32, ctx.dops.vop_fscale.get<float>() + f_base,
+      reinterpret_cast<float2*>(sout));
 }
 
 template <class Real, int PB>
@@ -2134,6 +2180,15 @@ void vlist_fft_t(Context& ctx, const double* ue, double* dc, Cplx<Real>* sin_, C
   const size_t sm_dn = F::tw_bytes + Gd * F::dn_grid_bytes;
   PVFMM_CUDA_CHECK(
       cudaFuncSetAttribute(ifft_dn_kernel<Real, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_dn));
+  // split-FP16 input spectra for the mixed form's tensor-core Hadamards
+  const double* qinv = nullptr;
+  if (sizeof(Real) == 4 && !(kin == 1 ? use_tc5(ctx) : use_simt3())) {
+    float* qs = ctx.qscale.as<float>(T.n_vsrc);
+    double* qi = ctx.qinv.as<double>(T.n_vsrc);
+    ++ctx.n_launch;
+    vsrc_scale_kernel<<<T.n_vsrc, 256, 0, s>>>(T.vsrc.get<int>(), T.child0.get<int>(), ue, ctx.ns * kin, qs, qi);
+    qinv = qi;
+  }
   // slabs of kz (the slowest frequency index): each slab's forward DFT rows,
   // products and inverse DFT contribution in turn (nslab = 1: all at once)
   for (int sl = 0; sl < nslab; ++sl) {
@@ -2143,7 +2198,7 @@ void vlist_fft_t(Context& ctx, const double* ue, double* dc, Cplx<Real>* sin_, C
     ++ctx.n_launch;
     fft_up_kernel<Real, M><<<T.n_vsrc * (ngrid_up / Gu), F::threads(Gu), sm_up, s>>>(
         kin, Gu, ngrid_up / Gu, T.vsrc.get<int>(), T.child0.get<int>(), ue, ctx.dops.fft_map.get<int>(), ctx.ns,
-        T.n_vsrc, kz0, nkz, sin_);
+        T.n_vsrc, kz0, nkz, qinv, sin_);
     if (sl == 0) ev(4);
     for (long p0 = 0; p0 < T.n_vtrg; p0 += chunk) {
       const long np = std::min(chunk, T.n_vtrg - p0);
@@ -2515,81 +2570,58 @@ void evaluate_impl(Context& ctx, const void* den_in, const void* dl_in, bool den
 
 }  // namespace
 
-// B fragments of hadamard_tc_kernel: for frequency f, offset o, lane (g, t)
-// and block (k-step s, n-tile nt): b0 = B[(j2, re)][(j1, pout)],
-// b1 = B[(j2, im)][(j1, pout)] with j2 = 2t + s, j1 = 4 nt + g/2,
-// pout = g % 2, where the real form of the complex block M = M[f][o][j1][j2]
-// is B[(j2,re)][(j1,re)] = Re M, B[(j2,im)][(j1,re)] = -Im M,
-// B[(j2,re)][(j1,im)] = Im M, B[(j2,im)][(j1,im)] = Re M.  Each value is
-// stored as [f][o][block (s, nt)][lane] float4 = (b0 hi, b1 hi, b0 lo, b1 lo),
-// hi = the value rounded to TF32, lo = the remainder rounded to TF32 (round
-// half away from zero, as cvt.rna), so that a warp's loads of one block are
-// consecutive.
-static float tf32_rna(float x) {
-  unsigned u;
-  std::memcpy(&u, &x, 4);
-  if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0x1000u) & 0xffffe000u;
-  float r;
-  std::memcpy(&r, &u, 4);
-  return r;
+// Exponents of the operators per frequency: fscale[f] = 2^(E - 14) with every
+// |re|, |im| of frequency f below 2^E, so that the fragments stay below 2^14.
+__global__ void __launch_bounds__(256) vop_scale_kernel(int n, const float2* __restrict__ vop,
+                                                        float* __restrict__ fscale) {
+  __shared__ float part[256];
+  float top = 0;
+  for (int i = threadIdx.x; i < n; i += 256) {
+    const float2 v = vop[(long)blockIdx.x * n + i];
+    top = fmaxf(top, fmaxf(fabsf(v.x), fabsf(v.y)));
+  }
+  part[threadIdx.x] = top;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 256; ++i) top = fmaxf(top, part[i]);
+    int e = 14;
+    if (top > 0) frexpf(top, &e);
+    fscale[blockIdx.x] = ldexpf(1.f, e - 14);
+  }
 }
 
-static void upload_vop_fragments(Context& ctx) {
-  const HostOperators& h = ctx.hops;
-  const int m = ctx.m, n3h = 4 * m * m * (m + 1);
-  std::vector<float> fr((size_t)n3h * 26 * 4 * 32 * 4);
-  auto split = [](float x, float& hi, float& lo) {
-    hi = tf32_rna(x);
-    lo = tf32_rna(x - hi);
-  };
-  for (int f = 0; f < n3h; ++f)
-    for (int o = 0; o < 26; ++o)
-      for (int lane = 0; lane < 32; ++lane) {
-        const int g = lane >> 2, t = lane & 3;
-        for (int s = 0; s < 2; ++s)
-          for (int nt = 0; nt < 2; ++nt) {
-            const int j2 = 2 * t + s, j1 = 4 * nt + (g >> 1), pout = g & 1;
-            const size_t src = ((((size_t)f * 26 + o) * 8 + j1) * 8 + j2) * 2;
-            const float mr = (float)h.vop[src], mi = (float)h.vop[src + 1];
-            const float b0 = pout == 0 ? mr : mi;   // from (j2, re)
-            const float b1 = pout == 0 ? -mi : mr;  // from (j2, im)
-            float* d = &fr[((((size_t)f * 26 + o) * 4 + s * 2 + nt) * 32 + lane) * 4];
-            split(b0, d[0], d[2]);
-            split(b1, d[1], d[3]);
-          }
-      }
-  float* dev = ctx.dops.vop_frag.as<float>(fr.size());
-  PVFMM_CUDA_CHECK(cudaMemcpyAsync(dev, fr.data(), fr.size() * sizeof(float), cudaMemcpyHostToDevice, ctx.stream));
-  PVFMM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
-}
-
-// B fragments of hadamard_tc3_kernel: for frequency f, offset o, output group
-// z (KOC components), block (k-step s = 2u + v, n-tile nt) and lane (g, t):
-// b0 = B[(e_in, re)][(e_out, re|im)], b1 = B[(e_in, im)][(e_out, re|im)] with
-// input element e_in = 8u + 2t + v = j2 * 3 + i, output element
-// e_out = 4 nt + g / 2 = j1 * KOC + c (component z KOC + c), re|im = g % 2;
-// stored as [f][o][z][block][lane] float4 = (b0 hi, b1 hi, b0 lo, b1 lo).
-// Built on the device from the FP32 operator blocks vop[f][o][j1][j2][i][c].
-__global__ void vop3_fragments_kernel(long n, int ko, int koc, const float2* __restrict__ vop,
-                                      float4* __restrict__ frag) {
+// B fragments of hadamard_tc_kernel and hadamard_tc3_kernel: for frequency f,
+// offset o, output group z (KOC components), block (k-step u, n-tile nt) and
+// lane (g, t), the operator entries of the input elements e = 8u + 2t (b0) and
+// e + 1 (b1), e = j2 * ki + i, onto column 8 nt + g (output element
+// e_out = 4 nt + g / 2 = j1 * KOC + c, component z KOC + c, re|im = g % 2):
+// b0 = (B[(e, re)], B[(e, im)]) with B[(e, re)][(e_out, re)] = Re M,
+// B[(e, im)][(e_out, re)] = -Im M, B[(e, re)][(e_out, im)] = Im M,
+// B[(e, im)][(e_out, im)] = Re M; divided by fscale[f] and stored as
+// [f][o][z][block][lane] uint4 = (b0 hi, b1 hi, b0 lo, b1 lo).  Built on the
+// device from the FP32 operator blocks vop[f][o][j1][j2][i][c].
+__global__ void vop_fragments_kernel(long n, int ki, int ko, int koc, const float2* __restrict__ vop,
+                                     const float* __restrict__ fscale, uint4* __restrict__ frag) {
   const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (idx >= n) return;
-  const int nnt = 2 * koc, nb = 6 * nnt, ngroups = ko / koc;
+  const int nnt = 2 * koc, nb = ki * nnt, ngroups = ko / koc;
   const int lane = (int)(idx % 32);
   const int blk = (int)(idx / 32 % nb);
-  const long fo = idx / 32 / nb / ngroups;  // f * 26 + o
   const int z = (int)(idx / 32 / nb % ngroups);
-  const int sk = blk / nnt, nt = blk % nnt;
-  const int g = lane >> 2, t = lane & 3, u = sk >> 1, v = sk & 1;
-  const int e_in = 8 * u + 2 * t + v, e_out = 4 * nt + g / 2, pout = g & 1;
-  const int j2 = e_in / 3, i = e_in % 3, j1 = e_out / koc, c = z * koc + e_out % koc;
-  const float2 mv = vop[((fo * 8 + j1) * 8 + j2) * 3 * ko + i * ko + c];
-  const float b0 = pout == 0 ? mv.x : mv.y;   // from (e_in, re)
-  const float b1 = pout == 0 ? -mv.y : mv.x;  // from (e_in, im)
-  unsigned h0, l0, h1, l1;
-  tf32_split(b0, h0, l0);
-  tf32_split(b1, h1, l1);
-  frag[idx] = make_float4(__uint_as_float(h0), __uint_as_float(h1), __uint_as_float(l0), __uint_as_float(l1));
+  const long fo = idx / 32 / nb / ngroups;  // f * 26 + o
+  const int u = blk / nnt, nt = blk % nnt;
+  const int g = lane >> 2, t = lane & 3;
+  const int e_out = 4 * nt + g / 2, pout = g & 1;
+  const int j1 = e_out / koc, c = z * koc + e_out % koc;
+  const float inv = 1.f / fscale[fo / 26];  // a power of two
+  unsigned hi[2], lo[2];
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    const int e = 8 * u + 2 * t + w, j2 = e / ki, i = e % ki;
+    const float2 mv = vop[(((fo * 8 + j1) * 8 + j2) * ki + i) * ko + c];
+    half_split((pout == 0 ? mv.x : mv.y) * inv, (pout == 0 ? -mv.y : mv.x) * inv, hi[w], lo[w]);
+  }
+  frag[idx] = make_uint4(hi[0], hi[1], lo[0], lo[1]);
 }
 
 // B fragments of hadamard_dmma3_kernel: for frequency f, offset o, output
@@ -2656,14 +2688,16 @@ static void upload_vop_dmma3_fragments(Context& ctx) {
   PVFMM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
 }
 
-static void upload_vop3_fragments(Context& ctx) {
+static void upload_vop_fragments(Context& ctx) {
   const HostOperators& h = ctx.hops;
   const int m = ctx.m, n3h = 4 * m * m * (m + 1);
-  const int ko = h.kout, koc = ko == 1 ? 1 : 3;
-  const long n = (long)n3h * 26 * (ko / koc) * (12 * koc) * 32;
-  float4* dev = ctx.dops.vop_frag.as<float4>(n);
-  ++ctx.n_launch;
-  vop3_fragments_kernel<<<ceil_div(n, 256L), 256, 0, ctx.stream>>>(n, ko, koc, ctx.dops.vop.get<float2>(), dev);
+  const int ki = h.kin, ko = h.kout, koc = ko == 1 ? 1 : 3;
+  const long n = (long)n3h * 26 * (ko / koc) * (ki * 2 * koc) * 32;
+  uint4* dev = ctx.dops.vop_frag.as<uint4>(n);
+  float* fs = ctx.dops.vop_fscale.as<float>(n3h);
+  ctx.n_launch += 2;
+  vop_scale_kernel<<<n3h, 256, 0, ctx.stream>>>(26 * 64 * ki * ko, ctx.dops.vop.get<float2>(), fs);
+  vop_fragments_kernel<<<ceil_div(n, 256L), 256, 0, ctx.stream>>>(n, ki, ko, koc, ctx.dops.vop.get<float2>(), fs, dev);
   PVFMM_CUDA_CHECK(cudaGetLastError());
   PVFMM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
 }
@@ -2749,7 +2783,6 @@ void upload_operators(Context& ctx) {
   if (ctx.precision == 0) upload_vec<double>(ctx.dops.vop, h.vop, s);
   else upload_vec<float>(ctx.dops.vop, h.vop, s);
   if (ctx.precision == 1 && ctx.ki.ke == 1) {
-    upload_vop_fragments(ctx);
     std::vector<float> lay;
     hadamard_tc5_operator_layout(h.vop, 4 * ctx.m * ctx.m * (ctx.m + 1), lay);
     float* dev = ctx.dops.vop_tc5.as<float>(lay.size());
@@ -2763,7 +2796,7 @@ void upload_operators(Context& ctx) {
   PVFMM_CUDA_CHECK(cudaMemcpyAsync(fm, h.fft_map.data(), h.fft_map.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   PVFMM_CUDA_CHECK(cudaMemcpyAsync(im, h.ifft_map.data(), h.ifft_map.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   PVFMM_CUDA_CHECK(cudaStreamSynchronize(s));
-  if (ctx.precision == 1 && ctx.ki.ke == 3) upload_vop3_fragments(ctx);  // from the uploaded FP32 vop
+  if (ctx.precision == 1) upload_vop_fragments(ctx);  // from the uploaded FP32 vop
   if (ctx.precision == 0 && ctx.ki.ke == 3) upload_vop_dmma3_fragments(ctx);  // from the uploaded FP64 vop
   if (ctx.precision == 0 && ctx.ki.ke == 1) upload_vop_dmma1_fragments(ctx);
 }

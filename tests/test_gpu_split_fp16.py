@@ -1,0 +1,57 @@
+"""The mixed form's split-FP16 V-list products (eval.cu, hadamard_tc_kernel
+and hadamard_tc3_kernel): scales, empty parents and partial tiles.
+
+Bars: the mixed form's 1e-6 against the plain form for scalar kernels; the
+vector kernels also cut the downward pseudo-inverse at FP32 level, so they are
+compared with the mixed form's own FP32 SIMT products (1e-6, the bar of that
+comparison in test_gpu_parity.py).  Powers of two scale every stored half, sum
+and output exactly, so scaled densities give bit-identical scaled outputs.
+"""
+import numpy as np
+import pytest
+
+import pvfmm_b200 as P
+
+pytestmark = pytest.mark.gpu
+
+KERNELS = [(P.FMMKernel.LaplacePotGrad, 8), (P.FMMKernel.StokesPressure, 4), (P.FMMKernel.StokesVelocity, 4)]
+
+
+def _ctx(kernel, m, precision=P.PRECISION_MIXED, leaf=30):
+    return P.FMMParticleContext(-1, leaf, m, kernel, precision=precision)
+
+
+def _rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("kernel,m", KERNELS)
+@pytest.mark.parametrize("k", [-70, 70])
+def test_power_of_two_densities_scale_the_output_exactly(kernel, m, k):
+    rng = np.random.default_rng(5)
+    x = rng.random(3 * 3001)
+    q = rng.standard_normal(3001 * P.KERNEL_DIMS[kernel][0])
+    ctx = _ctx(kernel, m)
+    a = ctx.evaluate(x, q, None, x, True)
+    b = ctx.evaluate(x, np.ldexp(q, k), None, x, False)
+    assert np.array_equal(b, np.ldexp(a, k))
+
+
+# 600 / 1500 / 5001 points: 1 V-list target parent below a full tile of 16,
+# a few tiles, several tiles per warp with a remainder
+@pytest.mark.parametrize("kernel,m", KERNELS)
+@pytest.mark.parametrize("n", [600, 1500, 5001])
+def test_empty_parents_and_partial_tiles(monkeypatch, kernel, m, n):
+    rng = np.random.default_rng(n)
+    pos = rng.random((n, 3))
+    q = rng.standard_normal((n, P.KERNEL_DIMS[kernel][0]))
+    q[pos[:, 0] < 0.5] = 0.0                        # parents whose spectra are all zero
+    q[pos[:, 0] > 0.9] *= 2.0 ** 30                 # and parents of a very different scale
+    x = pos.reshape(-1)
+    a = _ctx(kernel, m).evaluate(x, q.reshape(-1), None, x, True)
+    if P.KERNEL_DIMS[kernel][0] == 1:
+        b = _ctx(kernel, m, P.PRECISION_PLAIN).evaluate(x, q.reshape(-1), None, x, True)
+    else:
+        monkeypatch.setenv("PVFMM_B200_HADAMARD3", "simt")
+        b = _ctx(kernel, m).evaluate(x, q.reshape(-1), None, x, True)
+    assert _rel(a, b) < 1e-6
