@@ -72,18 +72,6 @@ __device__ __forceinline__ void image_shift(unsigned char code, double& cx, doub
   cz += (double)(code / 9) - 1.0;
 }
 
-// ---------------------------------------------------------------------------
-// Source tiles in shared memory and the per-thread evaluation loop.
-// ---------------------------------------------------------------------------
-template <class Real, int KS>
-struct Tile {
-  Real x[kNT], y[kNT], z[kNT], f[KS][kNT];
-  // FP32 tiles carry the rounding remainder of each coordinate, so that the
-  // difference target - source is as accurate as FP32 rounding of the
-  // difference itself (close pairs dominate the gradient kernels).
-  Real xl[sizeof(Real) == 4 ? kNT : 1], yl[sizeof(Real) == 4 ? kNT : 1], zl[sizeof(Real) == 4 ? kNT : 1];
-};
-
 // Target coordinate as (hi, lo) in Real.
 template <class Real>
 struct Pt {
@@ -99,127 +87,6 @@ __device__ __forceinline__ Pt<Real> make_pt(double x, double y, double z) {
   p.yl = (Real)(y - (double)p.y);
   p.zl = (Real)(z - (double)p.z);
   return p;
-}
-
-template <class Real, int KS>
-__device__ __forceinline__ void tile_store(Tile<Real, KS>& tl, int i, double x, double y, double z) {
-  tl.x[i] = (Real)x;
-  tl.y[i] = (Real)y;
-  tl.z[i] = (Real)z;
-  if constexpr (sizeof(Real) == 4) {
-    tl.xl[i] = (Real)(x - (double)tl.x[i]);
-    tl.yl[i] = (Real)(y - (double)tl.y[i]);
-    tl.zl[i] = (Real)(z - (double)tl.z[i]);
-  }
-}
-
-template <class Real, int KS>
-__device__ __forceinline__ void tile_diff(const Tile<Real, KS>& tl, int j, const Pt<Real>& p, Real& rx, Real& ry,
-                                          Real& rz) {
-  if constexpr (sizeof(Real) == 4) {
-    rx = (p.x - tl.x[j]) + (p.xl - tl.xl[j]);
-    ry = (p.y - tl.y[j]) + (p.yl - tl.yl[j]);
-    rz = (p.z - tl.z[j]) + (p.zl - tl.zl[j]);
-  } else {
-    rx = p.x - tl.x[j];
-    ry = p.y - tl.y[j];
-    rz = p.z - tl.z[j];
-  }
-}
-
-// Sums sources j = j0, j0+js, ... < n of the tile into acc (FP64).  Two
-// independent partial sums in Real give ILP; the tile sum is promoted to
-// FP64, so FP32 rounding never accumulates over more than one tile.
-template <class Real, int Ker, bool Surface1 = false>
-__device__ __forceinline__ void tile_sum(const Tile<Real, KerDims<Ker>::KS>& tl, int n, int j0, int js,
-                                         const Pt<Real>& p, double* acc) {
-  constexpr int KS = KerDims<Ker>::KS, KT = KerDims<Ker>::KT;
-  Real u0[KT], u1[KT];
-#pragma unroll
-  for (int k = 0; k < KT; ++k) u0[k] = u1[k] = 0;
-  int j = j0;
-  for (; j + js < n; j += 2 * js) {
-    Real f0[KS], f1[KS];
-#pragma unroll
-    for (int i = 0; i < KS; ++i) {
-      f0[i] = tl.f[i][j];
-      f1[i] = tl.f[i][j + js];
-    }
-    Real rx, ry, rz;
-    tile_diff(tl, j, p, rx, ry, rz);
-    ker_eval<Ker, Real, Surface1>(rx, ry, rz, f0, u0);
-    tile_diff(tl, j + js, p, rx, ry, rz);
-    ker_eval<Ker, Real, Surface1>(rx, ry, rz, f1, u1);
-  }
-  if (j < n) {
-    Real f0[KS];
-#pragma unroll
-    for (int i = 0; i < KS; ++i) f0[i] = tl.f[i][j];
-    Real rx, ry, rz;
-    tile_diff(tl, j, p, rx, ry, rz);
-    ker_eval<Ker, Real, Surface1>(rx, ry, rz, f0, u0);
-  }
-#pragma unroll
-  for (int k = 0; k < KT; ++k) acc[k] += (double)u0[k] + (double)u1[k];
-}
-
-// Work split of a block over a chunk of nc targets: thread t evaluates target
-// t % nc against the sources j == t / nc (mod G) of every tile.
-struct Split {
-  int nc, G, ti, g;
-  bool active;
-  __device__ explicit Split(int n_targets) {
-    nc = max(1, min(kNT, n_targets));
-    G = min(8, kNT / nc);
-    ti = threadIdx.x % nc;
-    g = threadIdx.x / nc;
-    active = g < G && ti < n_targets;
-  }
-};
-
-// Sources = sorted points [lo,hi) of a leaf whose centre is at offset (ox,oy,oz).
-template <class Real, int Ker, bool Surface1 = false>
-__device__ void point_sources(Tile<Real, KerDims<Ker>::KS>& tl, const double* __restrict__ sx,
-                              const double* __restrict__ sy, const double* __restrict__ sz,
-                              const double* __restrict__ den, int lo, int hi, double ox, double oy, double oz,
-                              const Split& sp, const Pt<Real>& pt, double* acc) {
-  constexpr int KS = KerDims<Ker>::KS;
-  for (int p0 = lo; p0 < hi; p0 += kNT) {
-    const int n = min(kNT, hi - p0);
-    __syncthreads();
-    if (threadIdx.x < n) {
-      const int p = p0 + threadIdx.x;
-      tile_store(tl, threadIdx.x, sx[p] + ox, sy[p] + oy, sz[p] + oz);
-#pragma unroll
-      for (int i = 0; i < KS; ++i) tl.f[i][threadIdx.x] = (Real)den[(long)p * KS + i];
-    }
-    __syncthreads();
-    if (sp.active) tile_sum<Real, Ker, Surface1>(tl, n, sp.g, sp.G, pt, acc);
-  }
-}
-
-// Adds the G partial sums of each target (deterministic order) and stores.
-template <int KT>
-__device__ void reduce_store(double (*red)[KT], const Split& sp, const double* acc, double scale, double* out,
-                             bool accumulate) {
-  __syncthreads();
-  if (sp.active)
-#pragma unroll
-    for (int k = 0; k < KT; ++k) red[threadIdx.x][k] = acc[k];
-  __syncthreads();
-  if (sp.active && sp.g == 0) {
-    double s[KT];
-#pragma unroll
-    for (int k = 0; k < KT; ++k) s[k] = red[sp.ti][k];
-    for (int g = 1; g < sp.G; ++g)
-#pragma unroll
-      for (int k = 0; k < KT; ++k) s[k] += red[g * sp.nc + sp.ti][k];
-#pragma unroll
-    for (int k = 0; k < KT; ++k) {
-      if (accumulate) out[sp.ti * KT + k] += s[k] * scale;
-      else out[sp.ti * KT + k] = s[k] * scale;
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -743,102 +610,111 @@ __global__ void __launch_bounds__(kNF, sizeof(Real) == 8       ? PVFMM_NEAR_MIN_
 }
 
 // ---------------------------------------------------------------------------
-// Sources -> check surface of a node, FP64.  mode 0 (S2U, fmm_pts.txx:
-// 2275-2637): node = sleaf[b], sources = its own points, output row b of
-// `out` scaled by scale*2^-depth (level factor of the check->equivalent
-// operator).  mode 1 (X, fmm_pts.txx:4444-4736): node = xtrg[b], sources =
-// the X list, added to DC[node].
+// Sources -> check surface of a node, FP64.  XList = false (S2U, fmm_pts.txx:
+// 2275-2637): node = nodes[b], sources = its own points, output row b of
+// `out` scaled by scale*2^(-deg depth) (level factor of the check->equivalent
+// operator).  XList = true (X, fmm_pts.txx:4444-4736): sources = the points of
+// the X list's leaves, output row = node.  accumulate: added to the row.
+//
+// One thread per (node, pair of check points k and k + ns/2; ns is even),
+// numbered through all nodes, so that every lane has work whatever ns and the
+// leaf sizes are.  The lanes of a warp mostly share a node and read its
+// sources as broadcasts from L1: four loads for two pairs, no shared memory
+// and no barrier.  Bound by the FP64 pipe (12 operations a Laplace pair).
+// LPS neighbouring lanes split the sources of one pair and add their sums in
+// a fixed order: 4 for X, whose few nodes have long lists, and for S2U when
+// one thread per pair would not fill the chip (surface_lanes).
+// Against one block per node with the sources in shared memory and two Newton
+// steps: 4M clustered points S2U with its products 3.15 -> 2.81 ms, X list
+// 0.48 -> 0.36 ms.
 // ---------------------------------------------------------------------------
-// mode 2: as mode 0, added to the row (the double-layer pass after the single
-// layer's).
-// Surface1 (mode 0 only): the check surface lies at least 1.2 half-widths
-// from every point of the leaf, so FP64 needs one Newton step (mixed form).
-template <int Ker, bool Surface1 = false>
+inline int surface_lanes(long n_pairs) { return n_pairs < 148L * 1024 ? 4 : 1; }
+
+template <int Ker, bool XList, int LPS>
 __global__ void __launch_bounds__(kNT) surface_check_kernel(
-    int mode, const int* __restrict__ nodes, const MKey* __restrict__ keys, const int* __restrict__ slo,
+    long n_thr, const int* __restrict__ nodes, const MKey* __restrict__ keys, const int* __restrict__ slo,
     const int* __restrict__ shi, const int* __restrict__ x_off, const int* __restrict__ x_list,
     const unsigned char* __restrict__ x_img, const double* __restrict__ sx, const double* __restrict__ sy,
-    const double* __restrict__ sz,
-    const double* __restrict__ den, const double* __restrict__ usurf, int ns, double rad, double scale, int deg,
-    double* __restrict__ out) {
-  constexpr int KT = KerDims<Ker>::KT;
-  __shared__ Tile<double, KerDims<Ker>::KS> tl;
-  __shared__ double red[kNT][KT];
-  const int b = blockIdx.x;
+    const double* __restrict__ sz, const double* __restrict__ den, const double* __restrict__ usurf, int ns,
+    double rad, double scale, int deg, bool accumulate, double* __restrict__ out) {
+  constexpr int KS = KerDims<Ker>::KS, KT = KerDims<Ker>::KT;
+  constexpr int NP = LPS == 1 && KT <= 3 ? 2 : 1;  // partial sums per check point (even and odd sources)
+  const int sub = threadIdx.x % LPS;
+  const long id = (blockIdx.x * (long)kNT + threadIdx.x) / LPS;
+  if (id >= n_thr) return;
+  const int nh = ns / 2;
+  const long b = id / nh;
+  const int k = (int)(id - b * nh);
   const int T = nodes[b];
   double cx, cy, cz, half;
   int dT;
   node_geom(keys[T], cx, cy, cz, half, dT);
   const double hr = half * rad;
-  const int dim = ns * KT;
-  double* o = mode != 1 ? out + (long)b * dim : out + (long)T * dim;
-  const double oscale = mode != 1 ? scale * ldexp(1.0, -deg * dT) : scale;
-  // a leaf's own sources (mode 0, 2) that fit one tile are staged once for
-  // every chunk of check points; a chunk of kNT points (one group) then writes
-  // its sums directly, with no block barrier
-  const int lo0 = slo[T], n0 = shi[T] - lo0;
-  if (mode != 1 && n0 <= kNT) {
-    if (threadIdx.x < n0) {
-      const int p = lo0 + threadIdx.x;
-      tile_store(tl, threadIdx.x, sx[p], sy[p], sz[p]);
+  double px[2], py[2], pz[2], acc[2][NP][KT];
 #pragma unroll
-      for (int i = 0; i < KerDims<Ker>::KS; ++i) tl.f[i][threadIdx.x] = den[(long)p * KerDims<Ker>::KS + i];
-    }
-    __syncthreads();
-    for (int c0 = 0; c0 < ns; c0 += kNT) {
-      const Split sp(ns - c0);
-      const int k = c0 + sp.ti;
-      double px = 0, py = 0, pz = 0;
-      if (sp.active) {
-        px = hr * usurf[k * 3 + 0];
-        py = hr * usurf[k * 3 + 1];
-        pz = hr * usurf[k * 3 + 2];
-      }
-      const Pt<double> pt = make_pt<double>(px, py, pz);
-      double acc[KT];
+  for (int h = 0; h < 2; ++h) {
+    px[h] = hr * usurf[(k + h * nh) * 3 + 0];
+    py[h] = hr * usurf[(k + h * nh) * 3 + 1];
+    pz[h] = hr * usurf[(k + h * nh) * 3 + 2];
 #pragma unroll
-      for (int c = 0; c < KT; ++c) acc[c] = 0;
-      if (sp.active) tile_sum<double, Ker, Surface1>(tl, n0, sp.g, sp.G, pt, acc);
-      if (sp.G == 1) {
-        if (sp.active)
+    for (int i = 0; i < NP; ++i)
 #pragma unroll
-          for (int c = 0; c < KT; ++c) {
-            double* dst = o + (c0 + sp.ti) * KT + c;
-            *dst = mode == 2 ? *dst + acc[c] * oscale : acc[c] * oscale;
-          }
-      } else {
-        reduce_store<KT>(red, sp, acc, oscale, o + c0 * KT, mode != 0);
-      }
-    }
-    return;
+      for (int c = 0; c < KT; ++c) acc[h][i][c] = 0;
   }
-  for (int c0 = 0; c0 < ns; c0 += kNT) {
-    const Split sp(ns - c0);
-    const int k = c0 + sp.ti;
-    double px = 0, py = 0, pz = 0;
-    if (sp.active) {
-      px = hr * usurf[k * 3 + 0];
-      py = hr * usurf[k * 3 + 1];
-      pz = hr * usurf[k * 3 + 2];
-    }
-    const Pt<double> pt = make_pt<double>(px, py, pz);
-    double acc[KT];
-#pragma unroll
-    for (int c = 0; c < KT; ++c) acc[c] = 0;
-    if (mode != 1) {
-      point_sources<double, Ker, Surface1>(tl, sx, sy, sz, den, slo[T], shi[T], 0, 0, 0, sp, pt, acc);
-    } else {
-      for (int q = x_off[T]; q < x_off[T + 1]; ++q) {
-        const int S = x_list[q];
-        double sxc, syc, szc, sh;
-        int dS;
-        node_geom(keys[S], sxc, syc, szc, sh, dS);
-        if (x_img) image_shift(x_img[q], sxc, syc, szc);
-        point_sources<double, Ker>(tl, sx, sy, sz, den, slo[S], shi[S], sxc - cx, syc - cy, szc - cz, sp, pt, acc);
+  // the points [lo, hi) of a leaf whose centre is at (ox, oy, oz)
+  auto points = [&](int lo, int hi, double ox, double oy, double oz) {
+    auto one = [&](int j, int i) {
+      double f[KS];
+      double x = __ldg(sx + j), y = __ldg(sy + j), z = __ldg(sz + j);
+      if constexpr (XList) {
+        x += ox;
+        y += oy;
+        z += oz;
       }
+#pragma unroll
+      for (int c = 0; c < KS; ++c) f[c] = __ldg(den + (long)j * KS + c);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) ker_eval<Ker, double>(px[h] - x, py[h] - y, pz[h] - z, f, acc[h][i]);
+    };
+    int j = lo + sub;
+    for (; j + NP <= hi; j += NP * LPS)
+#pragma unroll
+      for (int i = 0; i < NP; ++i) one(j + i, i);
+    if (NP > 1 && j < hi) one(j, 0);
+  };
+  if constexpr (XList) {
+    for (int q = x_off[T]; q < x_off[T + 1]; ++q) {
+      const int S = x_list[q];
+      double sxc, syc, szc, sh;
+      int dS;
+      node_geom(keys[S], sxc, syc, szc, sh, dS);
+      if (x_img) image_shift(x_img[q], sxc, syc, szc);
+      points(slo[S], shi[S], sxc - cx, syc - cy, szc - cz);
     }
-    reduce_store<KT>(red, sp, acc, oscale, o + c0 * KT, mode != 0);
+  } else {
+    points(slo[T], shi[T], 0, 0, 0);
   }
+  if constexpr (LPS > 1) {
+    const unsigned grp = ((1u << LPS) - 1) << (threadIdx.x % 32 / LPS * LPS);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < KT; ++c)
+#pragma unroll
+        for (int d = 1; d < LPS; d <<= 1) acc[h][0][c] += __shfl_xor_sync(grp, acc[h][0][c], d);
+    if (sub != 0) return;
+  }
+  const double oscale = XList ? scale : scale * ldexp(1.0, -deg * dT);
+  double* o = out + ((XList ? (long)T : b) * ns + k) * KT;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < KT; ++c) {
+      double v = acc[h][0][c];
+      if (NP > 1) v += acc[h][NP - 1][c];
+      double* dst = o + (long)h * nh * KT + c;
+      *dst = accumulate ? *dst + v * oscale : v * oscale;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2291,6 +2167,21 @@ void vlist(Context& ctx, const double* ue, double* dc, int kin, int kout, const 
   }
 }
 
+// S2U check potentials of all source leaves from the values `den` per point.
+template <int Ker>
+void launch_s2u(Context& ctx, const double* den, double scale, bool accumulate, double* uc) {
+  DevTree& T = ctx.tree;
+  const long n = T.n_sleaf * (ctx.ns / 2);
+  auto run = [&](auto kernel, int lanes) {
+    kernel<<<ceil_div(n * lanes, kNT), kNT, 0, ctx.stream>>>(
+        n, T.sleaf.get<int>(), T.key.get<MKey>(), T.src_lo.get<int>(), T.src_hi.get<int>(), nullptr, nullptr, nullptr,
+        T.sx.get<double>(), T.sy.get<double>(), T.sz.get<double>(), den, ctx.dops.usurf.get<double>(), ctx.ns, kRad1,
+        scale, ctx.ki.deg, accumulate, uc);
+  };
+  if (surface_lanes(n) == 4) run(surface_check_kernel<Ker, false, 4>, 4);
+  else run(surface_check_kernel<Ker, false, 1>, 1);
+}
+
 template <class Real, int KerS2T, int KerExp>
 void evaluate_impl(Context& ctx, const void* den_in, const void* dl_in, bool den_float, void* out, bool out_float) {
   DevTree& T = ctx.tree;
@@ -2389,15 +2280,11 @@ void evaluate_impl(Context& ctx, const void* den_in, const void* dl_in, bool den
     // V-list does not cancel those (one Newton step here raised the 4M-point
     // potential error from 3e-7 to 2.5e-6)
     if (has_sl)
-      surface_check_kernel<KerExp, false><<<T.n_sleaf, kNT, 0, s>>>(
-          0, T.sleaf.get<int>(), keys, slo, shi, nullptr, nullptr, nullptr, sx, sy, sz, den, usurf, ns, kRad1, kscale_exp, deg,
-          uc);
+      launch_s2u<KerExp>(ctx, den, kscale_exp, false, uc);
     if constexpr (KerDblExp >= 0) {
       if (has_dl) {
         ++ctx.n_launch;
-        surface_check_kernel<KerDblExp, false><<<T.n_sleaf, kNT, 0, s>>>(
-            has_sl ? 2 : 0, T.sleaf.get<int>(), keys, slo, shi, nullptr, nullptr, nullptr, sx, sy, sz, surf, usurf, ns, kRad1,
-            ker_scale(KerDblExp), deg, uc);
+        launch_s2u<KerDblExp>(ctx, surf, ker_scale(KerDblExp), has_sl, uc);
       }
     }
     // equivalent densities (uc UC2UE0) UC2UE1 straight into the leaves' rows of UE
@@ -2482,16 +2369,17 @@ void evaluate_impl(Context& ctx, const void* den_in, const void* dl_in, bool den
   // ---- X-list
   if (T.src_counted && T.n_xtrg > 0) {
     ++ctx.n_launch;
+    const long n_thr = T.n_xtrg * (ns / 2);
     if (has_sl)
-      surface_check_kernel<KerExp><<<T.n_xtrg, kNT, 0, s>>>(1, T.xtrg.get<int>(), keys, slo, shi, T.x_off.get<int>(),
-                                                             T.x_list.get<int>(), ximg, sx, sy, sz, den, usurf, ns, kRad0,
-                                                             kscale_exp, deg, dc);
+      surface_check_kernel<KerExp, true, 4><<<ceil_div(4 * n_thr, kNT), kNT, 0, s>>>(
+          n_thr, T.xtrg.get<int>(), keys, slo, shi, T.x_off.get<int>(), T.x_list.get<int>(), ximg, sx, sy, sz, den,
+          usurf, ns, kRad0, kscale_exp, deg, true, dc);
     if constexpr (KerDblExp >= 0) {
       if (has_dl) {
         ++ctx.n_launch;
-        surface_check_kernel<KerDblExp><<<T.n_xtrg, kNT, 0, s>>>(
-            1, T.xtrg.get<int>(), keys, slo, shi, T.x_off.get<int>(), T.x_list.get<int>(), ximg, sx, sy, sz, surf, usurf,
-            ns, kRad0, ker_scale(KerDblExp), deg, dc);
+        surface_check_kernel<KerDblExp, true, 4><<<ceil_div(4 * n_thr, kNT), kNT, 0, s>>>(
+            n_thr, T.xtrg.get<int>(), keys, slo, shi, T.x_off.get<int>(), T.x_list.get<int>(), ximg, sx, sy, sz, surf,
+            usurf, ns, kRad0, ker_scale(KerDblExp), deg, true, dc);
       }
     }
   }
