@@ -239,9 +239,9 @@ __device__ __forceinline__ void rec_sum2(const typename Vec16<Real>::type* tile,
 
 // ---------------------------------------------------------------------------
 // Packed FP32 pairs (add/sub/mul/fma .f32x2 of sm_100): the mixed form's near
-// field evaluates a source record against its thread's two targets in the two
-// halves of 64-bit registers, one instruction per operation for both targets
-// (the same round-to-nearest FP32 operations as two scalar evaluations).
+// field evaluates two sources against a target in the two halves of 64-bit
+// registers, one instruction per operation for both (the same
+// round-to-nearest FP32 operations as two scalar evaluations).
 // ---------------------------------------------------------------------------
 typedef unsigned long long f2_t;
 __device__ __forceinline__ f2_t f2_pack(float lo, float hi) {
@@ -273,14 +273,17 @@ __device__ __forceinline__ f2_t f2_fma(f2_t a, f2_t b, f2_t c) {
   return d;
 }
 
-// Kernels with a packed form (the others evaluate the two targets in turn).
+// Kernels with a packed form (the others evaluate one source at a time).
 template <int Ker>
 constexpr bool kHasPacked = Ker == kKerLaplace || Ker == kKerLaplaceGrad || Ker == kKerLaplacePG || Ker == kKerStokes;
 
-// ker_eval<Ker, float> for two targets at once: r = target - source per half,
-// f the source densities (the same in both halves).  1/r: one hardware
-// reciprocal square root per half (0 for r2 == 0) and one packed
-// Newton-Raphson step y <- y (3/2 - r2 y^2 / 2), as rsqrt_nr(float).
+// ker_eval<Ker, float> for two sources at once: r = target - source per half,
+// f the source densities.  1/r: one hardware reciprocal square root per half
+// (0 for r2 == 0) and one packed Newton-Raphson step, kept at three
+// operations as y (r2 y^2 - 3) = -2/r; the Laplace kernels sum with that
+// value, -2 / r and (-2 / r)^3 being powers of two times the terms
+// (packed_unit, taken out of the FP64 sums), and Stokes velocity, whose terms
+// mix, scales it back.
 template <int Ker>
 __device__ __forceinline__ void ker_eval_x2(f2_t rx, f2_t ry, f2_t rz, const f2_t* f, f2_t* u) {
   const f2_t r2 = f2_fma(rz, rz, f2_fma(ry, ry, f2_mul(rx, rx)));
@@ -291,17 +294,18 @@ __device__ __forceinline__ void ker_eval_x2(f2_t rx, f2_t ry, f2_t rz, const f2_
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
   ya = a > 0.f ? ya : 0.f;
   yb = b > 0.f ? yb : 0.f;
-  f2_t y = f2_pack(ya, yb);
-  const f2_t half = f2_pack(0.5f, 0.5f), three_half = f2_pack(1.5f, 1.5f);
-  y = f2_mul(y, f2_sub(three_half, f2_mul(f2_mul(half, r2), f2_mul(y, y))));
+  const f2_t y0 = f2_pack(ya, yb);
+  const f2_t e = f2_fma(f2_mul(r2, y0), y0, f2_pack(-3.f, -3.f));
   if constexpr (Ker == kKerLaplace) {
-    u[0] = f2_fma(y, f[0], u[0]);
+    u[0] = f2_fma(f2_mul(y0, e), f[0], u[0]);
   } else if constexpr (Ker == kKerLaplaceGrad) {
+    const f2_t y = f2_mul(y0, e);
     const f2_t fr3 = f2_mul(f2_mul(y, y), f2_mul(y, f[0]));
     u[0] = f2_fma(rx, fr3, u[0]);
     u[1] = f2_fma(ry, fr3, u[1]);
     u[2] = f2_fma(rz, fr3, u[2]);
   } else if constexpr (Ker == kKerLaplacePG) {
+    const f2_t y = f2_mul(y0, e);
     const f2_t fr = f2_mul(y, f[0]);
     const f2_t fr3 = f2_mul(f2_mul(y, y), fr);
     u[0] = f2_add(u[0], fr);
@@ -309,6 +313,7 @@ __device__ __forceinline__ void ker_eval_x2(f2_t rx, f2_t ry, f2_t rz, const f2_
     u[2] = f2_fma(ry, fr3, u[2]);
     u[3] = f2_fma(rz, fr3, u[3]);
   } else {  // Stokes velocity: u += (f + r (f.r) / r^2) / r
+    const f2_t y = f2_mul(f2_mul(y0, f2_pack(-0.5f, -0.5f)), e);
     const f2_t ip = f2_mul(f2_fma(f[2], rz, f2_fma(f[1], ry, f2_mul(f[0], rx))), f2_mul(y, y));
     u[0] = f2_fma(y, f2_fma(rx, ip, f[0]), u[0]);
     u[1] = f2_fma(y, f2_fma(ry, ip, f[1]), u[1]);
@@ -316,44 +321,106 @@ __device__ __forceinline__ void ker_eval_x2(f2_t rx, f2_t ry, f2_t rz, const f2_
   }
 }
 
-// rec_sum2 for FP32 records with the packed pair evaluation.
-template <int Ker, int TS = kTile>
-__device__ __forceinline__ void rec_sum2_x2(const float4* tile, int n, int j0, int js, const Pt<float>& pa,
-                                            const Pt<float>& pb, double (&acc)[2][KerDims<Ker>::KT]) {
+// The densities of the kernels with 1/r^3 terms are stored divided by 8, so
+// that those terms overflow no sooner than the kernel's own.  Component k of
+// the packed evaluation is packed_unit times the kernel's.
+template <int Ker>
+constexpr float kPackedDen = Ker == kKerLaplaceGrad || Ker == kKerLaplacePG ? 0.125f : 1.f;
+template <int Ker>
+__host__ __device__ constexpr double packed_unit(int k) {
+  return !kHasPacked<Ker> || Ker == kKerStokes ? 1.0
+         : Ker == kKerLaplace                  ? -2.0
+         : Ker == kKerLaplacePG && k == 0      ? -0.25
+                                               : -1.0;
+}
+
+// Records of the packed evaluation: two consecutive sources share one record
+// of pairs (v of the first, v of the second) for v = x y z f0 | xl yl zl f1 f2,
+// two pairs per 16-byte chunk, chunk-major.  A chunk loads as two packed
+// operands for either target, so no operand is duplicated into a pair in the
+// loop (with pairs of targets every source value was).
+template <int KS>
+struct PairRec {
+  static constexpr int NV = 6 + KS;
+  static constexpr int NC = (NV + 1) / 2;
+  __host__ __device__ static constexpr int F(int i) { return i == 0 ? 3 : 6 + i; }
+};
+
+// Sources 2j and 2j+1 (x, y, z, f of each; the densities times `den`).
+template <int KS, int TP>
+__device__ __forceinline__ void pair_store(float4* tile, int j, const double (&x)[2], const double (&y)[2],
+                                           const double (&z)[2], const double (&f)[2][KS], float den) {
+  using R = PairRec<KS>;
+  float v[2 * R::NC][2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    v[0][u] = (float)x[u];
+    v[1][u] = (float)y[u];
+    v[2][u] = (float)z[u];
+    v[4][u] = (float)(x[u] - (double)v[0][u]);
+    v[5][u] = (float)(y[u] - (double)v[1][u]);
+    v[6][u] = (float)(z[u] - (double)v[2][u]);
+#pragma unroll
+    for (int i = 0; i < KS; ++i) v[R::F(i)][u] = (float)f[u][i] * den;
+    if (R::NV & 1) v[R::NV][u] = 0.f;
+  }
+#pragma unroll
+  for (int c = 0; c < R::NC; ++c)
+    tile[c * TP + j] = make_float4(v[2 * c][0], v[2 * c][1], v[2 * c + 1][0], v[2 * c + 1][1]);
+}
+
+// Adds the pairs j = j0, j0+js, ... < n of the tile (TP pairs) to two targets
+// (FP64 accumulators, in packed_unit units).
+template <int Ker, int TP>
+__device__ __forceinline__ void pair_sum2(const float4* tile, int n, int j0, int js, const Pt<float>& pa,
+                                          const Pt<float>& pb, double (&acc)[2][KerDims<Ker>::KT]) {
   constexpr int KS = KerDims<Ker>::KS, KT = KerDims<Ker>::KT;
-  using R = Rec<float, KS>;
-  const f2_t px = f2_pack(pa.x, pb.x), py = f2_pack(pa.y, pb.y), pz = f2_pack(pa.z, pb.z);
-  const f2_t pxl = f2_pack(pa.xl, pb.xl), pyl = f2_pack(pa.yl, pb.yl), pzl = f2_pack(pa.zl, pb.zl);
+  using R = PairRec<KS>;
+  f2_t p[2][6];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const Pt<float>& t = q ? pb : pa;
+    const float w[6] = {t.x, t.y, t.z, t.xl, t.yl, t.zl};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) p[q][i] = f2_pack(w[i], w[i]);
+  }
   // FP32 partial sums run over 16 records at most before going to FP64
   const int step = 16 * js;
   for (int jb = j0; jb < n; jb += step) {
     const int jend = min(n, jb + step);
-    f2_t u[KT];
+    f2_t u[2][KT];
 #pragma unroll
-    for (int k = 0; k < KT; ++k) u[k] = 0ull;  // (0.f, 0.f)
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int k = 0; k < KT; ++k) u[q][k] = 0ull;  // (0.f, 0.f)
 #pragma unroll kNearUnroll
     for (int j = jb; j < jend; j += js) {
-      float v[R::NVP];
+      f2_t v[2 * R::NC];
 #pragma unroll
       for (int c = 0; c < R::NC; ++c) {
-        const float4 w = tile[c * TS + j];
-        memcpy(&v[c * R::PER], &w, 16);
+        const float4 w = tile[c * TP + j];
+        v[2 * c] = f2_pack(w.x, w.y);
+        v[2 * c + 1] = f2_pack(w.z, w.w);
       }
       f2_t f[KS];
 #pragma unroll
-      for (int i = 0; i < KS; ++i) f[i] = f2_pack(v[R::F(i)], v[R::F(i)]);
-      const f2_t rx = f2_add(f2_sub(px, f2_pack(v[0], v[0])), f2_sub(pxl, f2_pack(v[4], v[4])));
-      const f2_t ry = f2_add(f2_sub(py, f2_pack(v[1], v[1])), f2_sub(pyl, f2_pack(v[5], v[5])));
-      const f2_t rz = f2_add(f2_sub(pz, f2_pack(v[2], v[2])), f2_sub(pzl, f2_pack(v[6], v[6])));
-      ker_eval_x2<Ker>(rx, ry, rz, f, u);
+      for (int i = 0; i < KS; ++i) f[i] = v[R::F(i)];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const f2_t rx = f2_add(f2_sub(p[q][0], v[0]), f2_sub(p[q][3], v[4]));
+        const f2_t ry = f2_add(f2_sub(p[q][1], v[1]), f2_sub(p[q][4], v[5]));
+        const f2_t rz = f2_add(f2_sub(p[q][2], v[2]), f2_sub(p[q][5], v[6]));
+        ker_eval_x2<Ker>(rx, ry, rz, f, u[q]);
+      }
     }
 #pragma unroll
-    for (int k = 0; k < KT; ++k) {
-      float a, b;
-      f2_unpack(u[k], a, b);
-      acc[0][k] += (double)a;
-      acc[1][k] += (double)b;
-    }
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int k = 0; k < KT; ++k) {
+        float a, b;
+        f2_unpack(u[q][k], a, b);
+        acc[q][k] += (double)a + (double)b;
+      }
   }
 }
 
@@ -392,11 +459,13 @@ __global__ void __launch_bounds__(kNF, sizeof(Real) == 8       ? PVFMM_NEAR_MIN_
   constexpr int TILE = near_tile<Real, Ker>();  // source records per tile
   constexpr int RPT = TILE / kNF;                 // records each thread fetches per tile
   using V = typename Vec16<Real>::type;
-  __shared__ V tiles[2][Rec<Real, KS>::NC * TILE];
+  constexpr int TILE_V = kPacked ? PairRec<KS>::NC * (TILE / 2) : Rec<Real, KS>::NC * TILE;
+  __shared__ V tiles[2][TILE_V];
   // the FP64 D2T records of the mixed form come first and reuse the tiles
   // (a barrier separates their last read from the first tile store), and so
   // do the partial sums of the final fixed-order reduction
-  static_assert(Rec<double, KS>::NC * 16 <= 2 * Rec<Real, KS>::NC * (int)sizeof(V), "D2T records fit the tiles");
+  constexpr int TILE64 = Rec<double, KS>::NC * TILE <= 2 * TILE_V ? TILE : TILE / 2;
+  static_assert(Rec<double, KS>::NC * TILE64 <= 2 * TILE_V, "D2T records fit the tiles");
   double2* tile64 = reinterpret_cast<double2*>(&tiles[0][0]);
   static_assert(sizeof(tiles) >= sizeof(double) * kNF * TPT * KT, "reduction buffer larger than the tiles");
   double(*red)[TPT][KT] = reinterpret_cast<double(*)[TPT][KT]>(&tiles[0][0]);
@@ -441,15 +510,15 @@ __global__ void __launch_bounds__(kNF, sizeof(Real) == 8       ? PVFMM_NEAR_MIN_
       if (de) {
         const double hr = half * kRad1;
         const double* dens = de + (long)b * dim;
-        for (int k0 = 0; k0 < ns; k0 += TILE) {
-          const int n = min(TILE, ns - k0);
+        for (int k0 = 0; k0 < ns; k0 += TILE64) {
+          const int n = min(TILE64, ns - k0);
           __syncthreads();
           for (int i = threadIdx.x; i < n; i += kNF) {
             const int k = k0 + i;
             double f[KS];
 #pragma unroll
             for (int c = 0; c < KS; ++c) f[c] = dens[k * KS + c];
-            rec_store<double, KS, TILE>(tile64, i, hr * usurf[k * 3 + 0], hr * usurf[k * 3 + 1],
+            rec_store<double, KS, TILE64>(tile64, i, hr * usurf[k * 3 + 0], hr * usurf[k * 3 + 1],
                                         hr * usurf[k * 3 + 2], f);
           }
           __syncthreads();
@@ -458,9 +527,15 @@ __global__ void __launch_bounds__(kNF, sizeof(Real) == 8       ? PVFMM_NEAR_MIN_
             for (int h = 0; h < TPT / 2; ++h) {
               const Pt<double> pa64 = make_pt<double>(tx[tq[2 * h]], ty[tq[2 * h]], tz[tq[2 * h]]);
               const Pt<double> pb64 = make_pt<double>(tx[tq[2 * h + 1]], ty[tq[2 * h + 1]], tz[tq[2 * h + 1]]);
-              rec_sum2<double, Ker, true, TILE>(tile64, n, g, G, pa64, pb64,
+              rec_sum2<double, Ker, true, TILE64>(tile64, n, g, G, pa64, pb64,
                                           *reinterpret_cast<double(*)[2][KT]>(&acc[2 * h][0]));
             }
+        }
+        if constexpr (kPacked) {
+#pragma unroll
+          for (int q = 0; q < TPT; ++q)
+#pragma unroll
+            for (int k = 0; k < KT; ++k) acc[q][k] *= packed_unit<Ker>(k);
         }
       }
     }
@@ -526,13 +601,21 @@ __global__ void __launch_bounds__(kNF, sizeof(Real) == 8       ? PVFMM_NEAR_MIN_
       __syncthreads();
       const int total = start[ne];
       const int ntile = (total + TILE - 1) / TILE;
-      // records j = threadIdx.x + u * kNF of a tile, fetched one tile ahead
+      // records slot(u) of a tile, fetched one tile ahead
+      auto slot = [&](int u) { return kPacked ? RPT * (int)threadIdx.x + u : (int)threadIdx.x + u * kNF; };
       double rx_[RPT], ry_[RPT], rz_[RPT], rf_[RPT][KS];
       auto fetch = [&](int t) {
 #pragma unroll
         for (int u = 0; u < RPT; ++u) {
-          const int r = t * TILE + threadIdx.x + u * kNF;
-          if (r >= total) continue;
+          const int r = t * TILE + slot(u);
+          if (r >= total) {
+            if constexpr (kPacked) {  // a missing second source of a pair: density 0, off the leaf
+              rx_[u] = ry_[u] = rz_[u] = 1;
+#pragma unroll
+              for (int c = 0; c < KS; ++c) rf_[u][c] = 0;
+            }
+            continue;
+          }
           int lo = 0, hi = ne;  // largest s with start[s] <= r
           while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -563,20 +646,25 @@ __global__ void __launch_bounds__(kNF, sizeof(Real) == 8       ? PVFMM_NEAR_MIN_
       if (ntile > 0) fetch(0);
       for (int t = 0; t < ntile; ++t) {
         const int n = min(TILE, total - t * TILE);
+        if constexpr (kPacked) {
+          static_assert(RPT == 2, "a thread stores the two sources of a pair");
+          if (slot(0) < n) pair_store<KS, TILE / 2>(tiles[buf], threadIdx.x, rx_, ry_, rz_, rf_, kPackedDen<Ker>);
+        } else {
 #pragma unroll
-        for (int u = 0; u < RPT; ++u) {
-          const int j = threadIdx.x + u * kNF;
-          if (j < n) {
-            Real f[KS];
+          for (int u = 0; u < RPT; ++u) {
+            const int j = slot(u);
+            if (j < n) {
+              Real f[KS];
 #pragma unroll
-            for (int c = 0; c < KS; ++c) f[c] = (Real)rf_[u][c];
-            rec_store<Real, KS, TILE>(tiles[buf], j, rx_[u], ry_[u], rz_[u], f);
+              for (int c = 0; c < KS; ++c) f[c] = (Real)rf_[u][c];
+              rec_store<Real, KS, TILE>(tiles[buf], j, rx_[u], ry_[u], rz_[u], f);
+            }
           }
         }
         if (t + 1 < ntile) fetch(t + 1);
         __syncthreads();  // tiles[buf] complete; tiles[buf^1] no longer read (its readers passed this barrier)
         if (active) {
-          if constexpr (kPacked) rec_sum2_x2<Ker, TILE>(tiles[buf], n, g, G, pt[0], pt[1], acc);
+          if constexpr (kPacked) pair_sum2<Ker, TILE / 2>(tiles[buf], (n + 1) / 2, g, G, pt[0], pt[1], acc);
           else rec_sum2<Real, Ker, false, TILE>(tiles[buf], n, g, G, pt[0], pt[1], acc);
         }
         buf ^= 1;
@@ -602,6 +690,10 @@ __global__ void __launch_bounds__(kNF, sizeof(Real) == 8       ? PVFMM_NEAR_MIN_
 #pragma unroll
           for (int k = 0; k < KT; ++k) sum[k] += red[gg * nc + ti][q][k];
         const long o = (long)(t0 + c0 + ti + q * nc) * KT;
+        if constexpr (kPacked) {
+#pragma unroll
+          for (int k = 0; k < KT; ++k) sum[k] *= 1.0 / packed_unit<Ker>(k);
+        }
 #pragma unroll
         for (int k = 0; k < KT; ++k) pot[o + k] = kDbl ? pot[o + k] + sum[k] * scale : sum[k] * scale;
       }
