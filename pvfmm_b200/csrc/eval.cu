@@ -873,32 +873,145 @@ __global__ void __launch_bounds__(256) vsrc_scale_kernel(const int* __restrict__
   }
 }
 
+// cos and sin of 2 pi j / N for the DFTs, evaluated by the compiler from their
+// Taylor series after reduction to [0, pi/4]: the twiddles of the unrolled
+// transforms become literal operands (read from shared memory before).
+constexpr double taylor_trig(double x, bool sine) {
+  double term = sine ? x : 1.0, sum = term;
+  for (int k = sine ? 2 : 1; k < 26; k += 2) {
+    term *= -x * x / (k * (k + 1));
+    sum += term;
+  }
+  return sum;
+}
+constexpr double twiddle_cos(int j, int N) {  // cos(2 pi j / N)
+  j %= N;
+  if (j < 0) j += N;
+  if (2 * j > N) j = N - j;                            // cos is even
+  if (4 * j > N) return -twiddle_cos(N - 2 * j, 2 * N);  // cos(pi - x) = -cos x
+  if (8 * j > N) return taylor_trig(1.57079632679489661923 * (N - 4 * j) / N, true);
+  return taylor_trig(6.28318530717958647693 * j / N, false);
+}
+constexpr double twiddle_sin(int j, int N) { return twiddle_cos(4 * j - N, 4 * N); }  // cos(x - pi/2)
+template <class Real, int N>
+struct Twiddles {
+  Real c[N] = {}, s[N] = {};
+  constexpr Twiddles() {
+    for (int j = 0; j < N; ++j) {
+      c[j] = (Real)twiddle_cos(j, N);
+      s[j] = (Real)twiddle_sin(j, N);
+    }
+    // exact where a factor is 0 or +-1
+    c[0] = 1;
+    s[0] = 0;
+    if (N % 2 == 0) {
+      c[N / 2] = -1;
+      s[N / 2] = 0;
+    }
+    if (N % 4 == 0) {
+      c[N / 4] = 0;
+      s[N / 4] = 1;
+      c[3 * (N / 4)] = 0;
+      s[3 * (N / 4)] = -1;
+    }
+  }
+};
+
+// a += v (c + i s) for constants c, s (folded when they are 0 or 1)
+template <class Real>
+__device__ __forceinline__ void cmac(Cplx<Real>& a, const Cplx<Real>& v, Real c, Real s) {
+  if (c == (Real)1) {
+    a.re += v.re;
+    a.im += v.im;
+  } else if (c != (Real)0) {
+    a.re += v.re * c;
+    a.im += v.im * c;
+  }
+  if (s == (Real)1) {
+    a.re -= v.im;
+    a.im += v.re;
+  } else if (s == (Real)-1) {
+    a.re += v.im;
+    a.im -= v.re;
+  } else if (s != (Real)0) {
+    a.re -= v.im * s;
+    a.im += v.re * s;
+  }
+}
+template <class Real>
+__device__ __forceinline__ Cplx<Real> cadd(const Cplx<Real>& a, const Cplx<Real>& b) { return {a.re + b.re, a.im + b.im}; }
+template <class Real>
+__device__ __forceinline__ Cplx<Real> csub(const Cplx<Real>& a, const Cplx<Real>& b) { return {a.re - b.re, a.im - b.im}; }
+template <class Real>
+__device__ __forceinline__ Cplx<Real> cmuli(const Cplx<Real>& a) { return {-a.im, a.re}; }
+
+// Four outputs of the length-2M DFT of M values, X[k0 + j M/2], j = 0..3
+// (k0 < M/2): the values' classes y mod 4 are summed once, S_r = sum of
+// v[y] w^(k0 y) over y = r (mod 4), w = exp(-pi i / M), and since w^(y M/2) =
+// (-i)^y, X[k0 + j M/2] = sum_r (-i)^(j r) S_r.  A quarter of the products of
+// the plain sums.
+template <class Real, int M>
+__device__ __forceinline__ void dft_quad(const Cplx<Real> (&v)[M], int k0, Cplx<Real> (&x)[4]) {
+  constexpr Twiddles<Real, 2 * M> tw{};
+  Cplx<Real> S[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+#pragma unroll
+  for (int y = 0; y < M; ++y) cmac(S[y % 4], v[y], tw.c[(k0 * y) % (2 * M)], -tw.s[(k0 * y) % (2 * M)]);
+  const Cplx<Real> a = cadd(S[0], S[2]), b = csub(S[0], S[2]), c = cadd(S[1], S[3]), d = cmuli(csub(S[1], S[3]));
+  x[0] = cadd(a, c);
+  x[1] = csub(b, d);  // S0 - i S1 - S2 + i S3
+  x[2] = csub(a, c);
+  x[3] = cadd(b, d);
+}
+
+// Adds the inputs k0 + j M/2, j = 0..3 (u[j]) of the length-2M inverse DFT to
+// its outputs z = M .. 2M-1 (acc[zp], z = M + zp): W^(k z) = (-1)^k W^(k zp)
+// and W^(j zp M/2) = i^(j zp), so the four inputs are combined once per class
+// of zp mod 4.
+template <class Real, int M>
+__device__ __forceinline__ void idft_quad(const Cplx<Real> (&u)[4], int k0, Cplx<Real> (&acc)[M]) {
+  constexpr Twiddles<Real, 2 * M> tw{};
+  const Cplx<Real> a = cadd(u[0], u[2]), b = csub(u[0], u[2]), c = cadd(u[1], u[3]), d = cmuli(csub(u[1], u[3]));
+  // (-1)^(k0 + j M/2): M/2 odd flips the inputs j = 1, 3
+  constexpr bool kFlip = (M / 2) % 2 != 0;
+  const Cplx<Real> B[4] = {kFlip ? csub(a, c) : cadd(a, c), kFlip ? csub(b, d) : cadd(b, d),
+                           kFlip ? cadd(a, c) : csub(a, c), kFlip ? cadd(b, d) : csub(b, d)};
+#pragma unroll
+  for (int zp = 0; zp < M; ++zp) {
+    const int w = (k0 * zp) % (2 * M);
+    const Real sg = k0 % 2 ? (Real)-1 : (Real)1;
+    cmac(acc[zp], B[zp % 4], sg * tw.c[w], sg * tw.s[w]);
+  }
+}
+
 template <class Real, int M>
 struct FftSizes {
   static constexpr int N1 = 2 * M, NH = M + 1, M3 = M * M * M, N3H = N1 * N1 * NH;
-  // forward: grid g [M3] real, a1 [M*M][NH] complex, a2 [M][N1][NH] complex
-  // (+4 complex of padding per grid, so that the z-lines of 4 neighbouring
-  // grids fall into different banks)
+  // forward: a1 [M*M][NH] complex, a2 [M][N1][NH] complex (+4 complex of
+  // padding per grid, so that the z-lines of 4 neighbouring grids fall into
+  // different banks), the real grid [M3] in a2's memory
   static constexpr int A2S = M * N1 * NH + 4;
-  static constexpr size_t up_grid_bytes = sizeof(Real) * (M3 + 2 * (M * M * NH + A2S));
-  // inverse: b1 [M][N1][NH] (+4 padding), b2 [M][M][NH] complex, o [M3] real
+  static constexpr size_t up_grid_bytes = sizeof(Real) * 2 * (M * M * NH + A2S);
+  // inverse: b1 [M][N1][NH] (+4 padding), b2 [M][M][NH] complex, the real
+  // result [M3] in b1's memory
   static constexpr int B1S = M * N1 * NH + 4;
-  static constexpr size_t dn_grid_bytes = sizeof(Real) * (2 * (B1S + M * M * NH) + M3);
-  static constexpr size_t tw_bytes = sizeof(Real) * 2 * N1;
+  static constexpr size_t dn_grid_bytes = sizeof(Real) * 2 * (B1S + M * M * NH);
   static constexpr int threads(int G) { return ((8 * NH * G + 31) / 32) * 32; }  // one thread per line of the widest stage
 };
 
 // Each stage of the separable DFTs: one thread per input line; it loads the
-// line into registers once and writes every output along that axis
-// (twiddle index (k * x) mod N1 known at compile time, read as a broadcast).
-// Output layout: FP64 with ke == 1 writes the spectra piece-major,
-// spec[f][child][q] (16 bytes per child), so that the scalar Hadamard's
-// gathers over Morton-adjacent parents coalesce; FP32 with `qscale` (the
-// split-FP16 Hadamards) writes each value times 2^-E of its parent
-// (qscale[q] = 2^E) as FP16 hi + lo in the order of split_word; otherwise
-// rows spec[q][f][child*ke+comp].
+// line into registers once and writes every output along that axis (radix-4
+// sums along y and z, paired outputs kx and M - kx along x, literal twiddles).
+// Against plain sums with the twiddles in shared memory, piece-major FP64
+// spectra and 4-byte FP16 stores, 4M clustered points in the mixed form:
+// forward 1.73 -> 0.99 ms, inverse 1.62 -> 0.78 ms; 1M in FP64: 1.89 -> 0.64
+// and 0.95 -> 0.56 ms.  What bounds the forward one now is its 64-byte row
+// stores at the frequency-major stride.
+// Output layout: frequency-major rows (split_row) for the scalar FP64
+// Hadamards, spec[f][q][child], and for the split-FP16 ones (`qinv` given),
+// each value times 2^-E of its parent as FP16 hi + lo in the order of
+// split_word; otherwise rows spec[q][f][child*ke+comp].
 template <class Real, int M>
-__global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups, const int* __restrict__ vsrc,
+__global__ void __launch_bounds__(576) fft_up_kernel(int ke, int G, int ngroups, const int* __restrict__ vsrc,
                                                       const int* __restrict__ child0, const double* __restrict__ ue,
                                                       const int* __restrict__ fft_map, int ns, long n_q, int kz0,
                                                       int nkz, const double* __restrict__ qinv,
@@ -906,11 +1019,9 @@ __global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups,
   using F = FftSizes<Real, M>;
   constexpr int N1 = F::N1, NH = F::NH, M3 = F::M3, N3H = F::N3H, A2S = F::A2S;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Real* twr = reinterpret_cast<Real*>(smem_raw);
-  Real* twi = twr + N1;
-  Real* g = twi + N1;                                          // G * M3
-  Cplx<Real>* a1 = reinterpret_cast<Cplx<Real>*>(g + G * M3);  // G * M*M*NH
-  Cplx<Real>* a2 = a1 + G * M * M * NH;                        // G * A2S
+  Cplx<Real>* a1 = reinterpret_cast<Cplx<Real>*>(smem_raw);  // G * M*M*NH
+  Cplx<Real>* a2 = a1 + G * M * M * NH;                      // G * A2S
+  Real* g = reinterpret_cast<Real*>(a2);                     // G * M3, before a2 is written
   const int q = blockIdx.x / ngroups;
   const int gb = (blockIdx.x % ngroups) * G;
   const int ngrid = 8 * ke;
@@ -919,12 +1030,6 @@ __global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups,
   const int c0 = child0[P];
   const int dim = ns * ke;
   const double ascale = qinv ? qinv[q] : 1.0;
-  for (int j = threadIdx.x; j < N1; j += blockDim.x) {
-    double sn, cs;
-    sincospi(-2.0 * j / N1, &sn, &cs);
-    twr[j] = (Real)cs;
-    twi[j] = (Real)sn;
-  }
   for (int i = threadIdx.x; i < gn * M3; i += blockDim.x) g[i] = 0;
   __syncthreads();
   for (int i = threadIdx.x; i < gn * ns; i += blockDim.x) {
@@ -941,16 +1046,20 @@ __global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups,
     Real v[M];
 #pragma unroll
     for (int x = 0; x < M; ++x) v[x] = row[x];
+    // sums over even and odd x give both X[kx] = E + O and, since
+    // w^((M - kx) x) = (-1)^x conj(w^(kx x)), X[M - kx] = conj(E - O)
+    constexpr Twiddles<Real, N1> tw{};
 #pragma unroll
-    for (int kx = 0; kx < NH; ++kx) {
-      Real re = 0, im = 0;
+    for (int kx = 0; kx <= M / 2; ++kx) {
+      Cplx<Real> S[2] = {{0, 0}, {0, 0}};
 #pragma unroll
       for (int x = 0; x < M; ++x) {
         const int w = (kx * x) % N1;
-        re += v[x] * twr[w];
-        im += v[x] * twi[w];
+        if (tw.c[w] != (Real)0) S[x % 2].re += v[x] * tw.c[w];
+        if (tw.s[w] != (Real)0) S[x % 2].im -= v[x] * tw.s[w];
       }
-      a1[r * NH + kx] = {re, im};
+      a1[r * NH + kx] = cadd(S[0], S[1]);
+      if (kx < M - kx) a1[r * NH + M - kx] = {S[0].re - S[1].re, S[1].im - S[0].im};
     }
   }
   __syncthreads();
@@ -964,55 +1073,63 @@ __global__ void __launch_bounds__(288) fft_up_kernel(int ke, int G, int ngroups,
     for (int y = 0; y < M; ++y) v[y] = col[y * NH];
     Cplx<Real>* dst = a2 + gi * A2S + (z * N1) * NH + kx;
 #pragma unroll
-    for (int ky = 0; ky < N1; ++ky) {
-      Real re = 0, im = 0;
+    for (int k0 = 0; k0 < M / 2; ++k0) {
+      Cplx<Real> x[4];
+      dft_quad<Real, M>(v, k0, x);
 #pragma unroll
-      for (int y = 0; y < M; ++y) {
-        const int w = (ky * y) % N1;
-        re += v[y].re * twr[w] - v[y].im * twi[w];
-        im += v[y].re * twi[w] + v[y].im * twr[w];
-      }
-      dst[ky * NH] = {re, im};
+      for (int j = 0; j < 4; ++j) dst[(k0 + j * (M / 2)) * NH] = x[j];
     }
   }
   __syncthreads();
   // z -> kz: line = (gi, ky, kx), gi fastest; spectrum index f = kx + NH*(ky + N1*kz);
   // only the slab kz in [kz0, kz0+nkz) is written, at f - N1*NH*kz0
   Cplx<Real>* out = spec + (long)q * (N1 * NH * nkz) * ngrid;
-  for (int i = threadIdx.x; i < gn * N1 * NH; i += blockDim.x) {
+  // (every thread runs every step: neighbouring lanes exchange halves)
+  const int n_line = gn * N1 * NH;
+  const bool paired = sizeof(Real) == 4 && qinv && gn % 2 == 0 && gb % 2 == 0;
+  for (int i0 = 0; i0 < n_line; i0 += blockDim.x) {
+    const int i = i0 + threadIdx.x;
+    const bool in = i < n_line;
     const int gi = i % gn, l = i / gn;  // l = ky*NH + kx
-    const Cplx<Real>* col = a2 + gi * A2S + l;
+    const Cplx<Real>* col = a2 + (in ? gi * A2S + l : 0);
     Cplx<Real> v[M];
 #pragma unroll
     for (int z = 0; z < M; ++z) v[z] = col[z * N1 * NH];
 #pragma unroll
-    for (int kz = 0; kz < N1; ++kz) {
-      if (kz < kz0 || kz >= kz0 + nkz) continue;
-      Real re = 0, im = 0;
+    for (int k0 = 0; k0 < M / 2; ++k0) {
+      Cplx<Real> x[4];
+      dft_quad<Real, M>(v, k0, x);
 #pragma unroll
-      for (int z = 0; z < M; ++z) {
-        const int w = (kz * z) % N1;
-        re += v[z].re * twr[w] - v[z].im * twi[w];
-        im += v[z].re * twi[w] + v[z].im * twr[w];
-      }
-      const int f = l + N1 * NH * (kz - kz0);
-      if (sizeof(Real) == 8 && ke == 1) {
-        spec[((long)f * 8 + gb + gi) * n_q + q] = {re, im};
-      } else if (sizeof(Real) == 4 && qinv) {
-        unsigned hi, lo;
-        half_split((float)re, (float)im, hi, lo);
-        unsigned* w = reinterpret_cast<unsigned*>(spec) + split_row(f, q, n_q) * (2 * ngrid) + split_word(gb + gi);
-        w[0] = hi;
-        w[2] = lo;
-      } else {
-        out[(long)f * ngrid + gb + gi] = {re, im};
+      for (int j = 0; j < 4; ++j) {
+        const int kz = k0 + j * (M / 2);
+        if (kz < kz0 || kz >= kz0 + nkz) continue;
+        const int f = l + N1 * NH * (kz - kz0);
+        if (sizeof(Real) == 4 && qinv) {
+          unsigned hi, lo;
+          half_split((float)x[j].re, (float)x[j].im, hi, lo);
+          unsigned* row = reinterpret_cast<unsigned*>(spec) + split_row(f, q, n_q) * (2 * ngrid);
+          if (paired) {  // elements e, e + 1 of a 16-byte piece: (hi, hi) from the even lane, (lo, lo) from the odd one
+            const bool odd = gi & 1;
+            const unsigned got = __shfl_xor_sync(0xffffffffu, odd ? hi : lo, 1);
+            if (in)
+              *reinterpret_cast<uint2*>(row + split_word((gb + gi) & ~1) + (odd ? 2 : 0)) =
+                  odd ? make_uint2(got, lo) : make_uint2(hi, got);
+          } else if (in) {
+            unsigned* w = row + split_word(gb + gi);
+            w[0] = hi;
+            w[2] = lo;
+          }
+        } else if (in) {
+          if (sizeof(Real) == 8 && ke == 1) spec[split_row(f, q, n_q) * 8 + gb + gi] = x[j];
+          else out[(long)f * ngrid + gb + gi] = x[j];
+        }
       }
     }
   }
 }
 
 template <class Real, int M>
-__global__ void __launch_bounds__(288) ifft_dn_kernel(int ke, int G, int ngroups, const int* __restrict__ vtrg,
+__global__ void __launch_bounds__(576) ifft_dn_kernel(int ke, int G, int ngroups, const int* __restrict__ vtrg,
                                                        const int* __restrict__ child0, const MKey* __restrict__ keys,
                                                        const Cplx<Real>* __restrict__ spec,
                                                        const int* __restrict__ ifft_map, int ns, int deg, int kz0,
@@ -1020,12 +1137,10 @@ __global__ void __launch_bounds__(288) ifft_dn_kernel(int ke, int G, int ngroups
   using F = FftSizes<Real, M>;
   constexpr int N1 = F::N1, NH = F::NH, M3 = F::M3, N3H = F::N3H;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Real* twr = reinterpret_cast<Real*>(smem_raw);
-  Real* twi = twr + N1;
   constexpr int B1S = F::B1S;
-  Cplx<Real>* b1 = reinterpret_cast<Cplx<Real>*>(twi + N1);  // G * B1S
+  Cplx<Real>* b1 = reinterpret_cast<Cplx<Real>*>(smem_raw);  // G * B1S
   Cplx<Real>* b2 = b1 + G * B1S;                             // G * M*M*NH
-  Real* o = reinterpret_cast<Real*>(b2 + G * M * M * NH);    // G * M3
+  Real* o = reinterpret_cast<Real*>(b1);                     // G * M3, once b1 has been read
   const int vt = blockIdx.x / ngroups;
   const int gb = (blockIdx.x % ngroups) * G;
   const int ngrid = 8 * ke;
@@ -1036,13 +1151,6 @@ __global__ void __launch_bounds__(288) ifft_dn_kernel(int ke, int G, int ngroups
   decode_key(keys[P], X, Y, Z, dP);
   const double lscale = ldexp(1.0, deg * ((int)dP + 1));  // 2^(trg_scal * level of the children)
   const int dim = ns * ke;
-  for (int j = threadIdx.x; j < N1; j += blockDim.x) {
-    double sn, cs;
-    sincospi(2.0 * j / N1, &sn, &cs);  // inverse twiddles
-    twr[j] = (Real)cs;
-    twi[j] = (Real)sn;
-  }
-  __syncthreads();
   const Cplx<Real>* in = spec + (long)vt * (N1 * NH * nkz) * ngrid + gb;
   // kz -> z in [M, 2M): line = (gi, ky, kx) read straight from the spectrum
   // row of the parent (gi fastest: neighbouring threads read neighbouring
@@ -1050,57 +1158,63 @@ __global__ void __launch_bounds__(288) ifft_dn_kernel(int ke, int G, int ngroups
   // slab's frequencies alone is added into dc (the transform is linear).
   for (int i = threadIdx.x; i < gn * N1 * NH; i += blockDim.x) {
     const int gi = i % gn, l = i / gn;  // l = ky*NH + kx
-    Cplx<Real> v[N1];
+    Cplx<Real> acc[M] = {};
 #pragma unroll
-    for (int kz = 0; kz < N1; ++kz)
-      v[kz] = (kz >= kz0 && kz < kz0 + nkz) ? in[(long)(l + N1 * NH * (kz - kz0)) * ngrid + gi] : Cplx<Real>{0, 0};
+    for (int k0 = 0; k0 < M / 2; ++k0) {
+      Cplx<Real> u[4];
 #pragma unroll
-    for (int zp = 0; zp < M; ++zp) {
-      Real re = 0, im = 0;
-#pragma unroll
-      for (int kz = 0; kz < N1; ++kz) {
-        const int w = (kz * (M + zp)) % N1;
-        re += v[kz].re * twr[w] - v[kz].im * twi[w];
-        im += v[kz].re * twi[w] + v[kz].im * twr[w];
+      for (int j = 0; j < 4; ++j) {
+        const int kz = k0 + j * (M / 2);
+        u[j] = (kz >= kz0 && kz < kz0 + nkz) ? in[(long)(l + N1 * NH * (kz - kz0)) * ngrid + gi] : Cplx<Real>{0, 0};
       }
-      b1[gi * B1S + zp * N1 * NH + l] = {re, im};
+      idft_quad<Real, M>(u, k0, acc);
     }
+#pragma unroll
+    for (int zp = 0; zp < M; ++zp) b1[gi * B1S + zp * N1 * NH + l] = acc[zp];
   }
   __syncthreads();
   // ky -> y in [M, 2M): line = (gi, zp, kx), kx fastest
   for (int i = threadIdx.x; i < gn * M * NH; i += blockDim.x) {
     const int kx = i % NH, zg = i / NH;  // zg = gi*M + zp
     const Cplx<Real>* col = b1 + (zg / M) * B1S + ((zg % M) * N1) * NH + kx;
-    Cplx<Real> v[N1];
+    Cplx<Real> acc[M] = {};
 #pragma unroll
-    for (int ky = 0; ky < N1; ++ky) v[ky] = col[ky * NH];
+    for (int k0 = 0; k0 < M / 2; ++k0) {
+      Cplx<Real> u[4];
 #pragma unroll
-    for (int yp = 0; yp < M; ++yp) {
-      Real re = 0, im = 0;
-#pragma unroll
-      for (int ky = 0; ky < N1; ++ky) {
-        const int w = (ky * (M + yp)) % N1;
-        re += v[ky].re * twr[w] - v[ky].im * twi[w];
-        im += v[ky].re * twi[w] + v[ky].im * twr[w];
-      }
-      b2[(zg * M + yp) * NH + kx] = {re, im};
+      for (int j = 0; j < 4; ++j) u[j] = col[(k0 + j * (M / 2)) * NH];
+      idft_quad<Real, M>(u, k0, acc);
     }
+#pragma unroll
+    for (int yp = 0; yp < M; ++yp) b2[(zg * M + yp) * NH + kx] = acc[yp];
   }
   __syncthreads();
   // kx -> x in [M, 2M), c2r: line = (gi, zp, yp)
   for (int r = threadIdx.x; r < gn * M * M; r += blockDim.x) {
     const Cplx<Real>* row = b2 + r * NH;
-    Cplx<Real> v[NH];
+    // y[xp] = sum over kx of (2 for 0 < kx < M) (-1)^kx Re(v[kx] W^(kx xp));
+    // kx and M - kx share cos and sin up to the sign (-1)^xp
+    constexpr Twiddles<Real, N1> tw{};
+    Cplx<Real> even[M / 2], odd[M / 2];
 #pragma unroll
-    for (int kx = 0; kx < NH; ++kx) v[kx] = row[kx];
+    for (int kx = 0; kx < M / 2; ++kx) {
+      const Cplx<Real> p = row[kx], m = row[M - kx];
+      const Real f = (kx % 2 ? (Real)-1 : (Real)1) * (kx == 0 ? (Real)1 : (Real)2);
+      even[kx] = {f * (p.re + m.re), f * (p.im - m.im)};
+      odd[kx] = {f * (p.re - m.re), f * (p.im + m.im)};
+    }
+    const Cplx<Real> mid = row[M / 2];
 #pragma unroll
     for (int xp = 0; xp < M; ++xp) {
-      Real acc = 0;
+      // the middle frequency: W^(M xp / 2) = i^xp, (-1)^(M/2), weight 2
+      const Real f = ((M / 2) % 2 ? (Real)-1 : (Real)1) * (xp % 4 < 2 ? (Real)2 : (Real)-2);
+      Real acc = xp % 2 ? -f * mid.im : f * mid.re;
 #pragma unroll
-      for (int kx = 0; kx < NH; ++kx) {
-        const int w = (kx * (M + xp)) % N1;
-        const Real t = v[kx].re * twr[w] - v[kx].im * twi[w];
-        acc += (kx == 0 || 2 * kx == N1) ? t : (Real)2 * t;
+      for (int kx = 0; kx < M / 2; ++kx) {
+        const int w = (kx * xp) % N1;
+        const Cplx<Real>& t = xp % 2 ? odd[kx] : even[kx];
+        if (tw.c[w] != (Real)0) acc += t.re * tw.c[w];
+        if (tw.s[w] != (Real)0) acc -= t.im * tw.s[w];
       }
       o[r * M + xp] = acc;
     }
@@ -1218,9 +1332,8 @@ __global__ void __launch_bounds__(128) hadamard_kernel(int n3h, long n_vtrg, lon
 // straight from global memory (L2) into registers, one offset ahead of the one
 // it multiplies, so shared memory holds only the 26 operator blocks of the
 // block's frequency (read as 16-byte broadcasts).  The input spectra are
-// piece-major (IN[f][piece][Q]): the neighbours Q_o(P) of the Morton-ordered
-// parents of a warp are mostly adjacent, so each 16-byte gather of a warp
-// coalesces.  Offsets that none of the thread's parents has are skipped.
+// frequency-major rows (split_row).  Offsets that none of the thread's
+// parents has are skipped.
 template <class Real, int PB>
 __global__ void __launch_bounds__(128, 4) hadamard_rd_kernel(int n3h, long n_vtrg, long vt_stride, long n_vsrc,
                                                              const int* __restrict__ vtab,
@@ -1261,9 +1374,9 @@ __global__ void __launch_bounds__(128, 4) hadamard_rd_kernel(int n3h, long n_vtr
       const int q = pin[k] ? __ldg(vtab + (long)o * vt_stride + prow[k]) : -1;
       if (q >= 0) {
         mask |= 1u << k;
-        const V* r = reinterpret_cast<const V*>(spec_in) + (long)f * NV * n_vsrc + q;
+        const V* r = reinterpret_cast<const V*>(spec_in) + split_row(f, q, n_vsrc) * NV;
 #pragma unroll
-        for (int v = 0; v < NV; ++v) x[k][v] = __ldg(r + (long)v * n_vsrc);
+        for (int v = 0; v < NV; ++v) x[k][v] = __ldg(r + v);
       } else {
 #pragma unroll
         for (int v = 0; v < NV; ++v) memset(&x[k][v], 0, 16);
@@ -1814,13 +1927,14 @@ __global__ void __launch_bounds__(32 * kDmWarps, 2)
 // FP64 tensor cores: per frequency the real GEMM OUT[P][(j1, re|im)] +=
 // sum_o IN[Q_o(P)][(j2, re|im)] B_o[..][..] with K = N = 16 (4 k-steps, 2
 // n-tiles of mma.sync m8n8k4 .f64).  A warp owns MT tiles of 8 target parents;
-// with the K order k-step s, column t -> child 2t + s/2, re|im = s % 2, lane
-// (g, t) needs children 2t and 2t+1 of row g: two 16-byte pieces of the
-// piece-major input spectra (IN[f][child][Q], so the gathers of Morton-close
-// parents coalesce), gathered from L2 two offsets ahead.  A block stages its
+// with the K order k-step s, column t -> child t + 4 (s/2), re|im = s % 2, lane
+// (g, t) needs children t and t+4 of row g: two 16-byte pieces of its 128-byte
+// row of the frequency-major input spectra (four lanes read 64 contiguous
+// bytes), gathered from L2 two offsets ahead.  A block stages its
 // frequency's B fragments (26 offsets, 53 KB) once and walks `chunks` chunks
 // of target parents; each warp walks only the offsets occupied for one of its
-// parents.
+// parents.  Frequency-major rows instead of one 16-byte piece per child and
+// parent: 1M clustered points (m = 8) 6.35 -> 4.43 ms.
 // ---------------------------------------------------------------------------
 constexpr int kDm1Warps = 8;
 
@@ -1841,7 +1955,7 @@ __global__ void __launch_bounds__(32 * kDm1Warps, 2)
     double2* dst = reinterpret_cast<double2*>(Bs1);
     for (int i = threadIdx.x; i < 26 * 8 * 16; i += 32 * kDm1Warps) dst[i] = __ldg(src + i);
   }
-  const double2* in0 = spec_in + ((long)f * 8 + 2 * t) * n_vsrc;  // child 2t; child 2t+1 at + n_vsrc
+  const double2* in0 = spec_in + split_row(f, 0, n_vsrc) * 8 + t;  // row q: in0[8 q] (child t), in0[8 q + 4]
   for (int c = 0; c < chunks; ++c) {
     const long pb = ((long)blockIdx.x * chunks + c) * NP;
     if (pb >= n_vtrg) break;
@@ -1867,8 +1981,8 @@ __global__ void __launch_bounds__(32 * kDm1Warps, 2)
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         const int q = qs[o * NP + w0 + mt * 8 + g];
-        x[mt][0] = q >= 0 ? __ldg(in0 + q) : make_double2(0.0, 0.0);
-        x[mt][1] = q >= 0 ? __ldg(in0 + n_vsrc + q) : make_double2(0.0, 0.0);
+        x[mt][0] = q >= 0 ? __ldg(in0 + (long)q * 8) : make_double2(0.0, 0.0);
+        x[mt][1] = q >= 0 ? __ldg(in0 + (long)q * 8 + 4) : make_double2(0.0, 0.0);
       }
     };
     auto compute = [&](int o, const double2 (&x)[MT][2]) {
@@ -2096,13 +2210,14 @@ void upload_vec(DevBuf& b, const std::vector<double>& v, cudaStream_t s) {
   PVFMM_CUDA_CHECK(cudaStreamSynchronize(s));
 }
 
-// Largest divisor G of ngrid with fixed + G*per_grid <= budget and at most
-// 288 threads (the DFT kernels' launch bound) for threads(G) (at least 1).
+// Grids per block of the DFT kernels: the largest divisor G of ngrid with
+// G*per_grid <= budget and at most max_threads for threads(G) (at least 1;
+// the kernels are bounded to 576 threads).
 template <class F>
-int grids_per_block(size_t per_grid, size_t fixed, int ngrid, size_t budget) {
+int grids_per_block(size_t per_grid, int ngrid, size_t budget, int max_threads) {
   int best = 1;
   for (int G = 1; G <= ngrid; ++G)
-    if (ngrid % G == 0 && fixed + G * per_grid <= budget && F::threads(G) <= 288) best = G;
+    if (ngrid % G == 0 && G * per_grid <= budget && F::threads(G) <= max_threads) best = G;
   return best;
 }
 
@@ -2141,11 +2256,18 @@ void vlist_fft_t(Context& ctx, const double* ue, double* dc, Cplx<Real>* sin_, C
   auto s = ctx.stream;
   using F = FftSizes<Real, M>;
   const int ngrid_up = 8 * kin, ngrid_dn = 8 * kout;
-  const int Gu = grids_per_block<F>(F::up_grid_bytes, F::tw_bytes, ngrid_up, 64 * 1024);
-  const size_t sm_up = F::tw_bytes + Gu * F::up_grid_bytes;
+  // two blocks of 112 KB share an SM: the FP32 scalar DFTs of m = 8 take all 8
+  // children and so write (read) whole 64-byte rows of the spectra; forward,
+  // 4M clustered points, 0.99 ms against 1.30 ms with 4 children in 60 KB.
+  // The inverse gains only for those (0.85 -> 0.78 ms; the others are slower
+  // in large blocks: 1M Stokes m = 6 0.34 ms in 288 threads, 0.40 in 448).
+  const int Gu = grids_per_block<F>(F::up_grid_bytes, ngrid_up, 112 * 1024, 576);
+  const size_t sm_up = Gu * F::up_grid_bytes;
   PVFMM_CUDA_CHECK(cudaFuncSetAttribute(fft_up_kernel<Real, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_up));
-  const int Gd = grids_per_block<F>(F::dn_grid_bytes, F::tw_bytes, ngrid_dn, 80 * 1024);
-  const size_t sm_dn = F::tw_bytes + Gd * F::dn_grid_bytes;
+  const bool rows = sizeof(Real) == 4 && ngrid_dn == 8 && 8 * F::dn_grid_bytes <= 112 * 1024;
+  const int Gd = rows ? grids_per_block<F>(F::dn_grid_bytes, ngrid_dn, 112 * 1024, 576)
+                      : grids_per_block<F>(F::dn_grid_bytes, ngrid_dn, 80 * 1024, 288);
+  const size_t sm_dn = Gd * F::dn_grid_bytes;
   PVFMM_CUDA_CHECK(
       cudaFuncSetAttribute(ifft_dn_kernel<Real, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_dn));
   // split-FP16 input spectra for the mixed form's tensor-core Hadamards
@@ -2632,7 +2754,7 @@ __global__ void vop_dmma3_fragments_kernel(long n, int ko, int koc, const double
 
 // B fragments of hadamard_dmma1_kernel: for frequency f, offset o, block
 // (k-step s, n-tile nt) and lane (g, t): b = B[k][n] with k = (child
-// 2t + s/2, re|im s % 2) and n = 8 nt + g (child 4 nt + g/2, re|im g % 2);
+// t + 4 (s/2), re|im s % 2) and n = 8 nt + g (child 4 nt + g/2, re|im g % 2);
 // stored as [f][o][s][nt][lane] doubles.
 __global__ void vop_dmma1_fragments_kernel(long n, const double2* __restrict__ vop, double* __restrict__ frag) {
   const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -2640,7 +2762,7 @@ __global__ void vop_dmma1_fragments_kernel(long n, const double2* __restrict__ v
   const int lane = (int)(idx % 32), nt = (int)(idx / 32 % 2), sk = (int)(idx / 64 % 4);
   const long fo = idx / 256;  // f * 26 + o
   const int g = lane >> 2, t = lane & 3;
-  const int j2 = 2 * t + (sk >> 1), pin = sk & 1, j1 = 4 * nt + g / 2, pout = g & 1;
+  const int j2 = t + 4 * (sk >> 1), pin = sk & 1, j1 = 4 * nt + g / 2, pout = g & 1;
   const double2 mv = vop[(fo * 8 + j1) * 8 + j2];
   frag[idx] = pin == 0 ? (pout == 0 ? mv.x : mv.y) : (pout == 0 ? -mv.y : mv.x);
 }
