@@ -120,6 +120,9 @@ struct Context {
   DevBuf io_dl;
   DevBuf stat;            // small status / reduction buffer
   DevBuf t[24];           // temporaries of the tree build, reused across calls
+  DevBuf seed;            // sorted keys of the initial tree's seed grid (n_seed of them)
+  long n_seed = 0;
+  bool seed_float = false;  // precision it was formed in
   std::vector<DevBuf> lvlR, lvlS;  // per-level internal-node keys (refined / balanced)
   long n_launch = 0;      // own kernels launched since context creation
   std::vector<float> stage_ms;

@@ -190,11 +190,9 @@ __global__ void make_children(const MKey* __restrict__ cur, const int* __restric
 // clipped to the unit box; per axis these are parent(x) and the parent on the
 // side of x within its parent.  Invalid candidates get the sentinel key.
 // periodic: the mask of periodic axes (bit 0 x, bit 1 y, bit 2 z; 0 = free space)
-__global__ void nbr_parents(const MKey* __restrict__ S, long n, int d, int periodic, MKey* __restrict__ out) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__device__ __forceinline__ void parent_candidates(const MKey& key, int d, int periodic, MKey (&out)[8]) {
   unsigned int q[3], dd;
-  decode_key(S[i], q[0], q[1], q[2], dd);
+  decode_key(key, q[0], q[1], q[2], dd);
   const unsigned int w = kTwo30 >> d;
   const unsigned int pmask = ~((kTwo30 >> (d - 1)) - 1u);
   long cand[3][2];
@@ -209,9 +207,17 @@ __global__ void nbr_parents(const MKey* __restrict__ S, long n, int d, int perio
   }
   for (int c = 0; c < 8; ++c) {
     const long x = cand[0][c & 1], y = cand[1][(c >> 1) & 1], z = cand[2][(c >> 2) & 1];
-    out[i * 8 + c] = (x < 0 || y < 0 || z < 0) ? MKey{~0ULL, ~0u, 0}
-                                               : make_key((unsigned int)x, (unsigned int)y, (unsigned int)z, d - 1);
+    out[c] = (x < 0 || y < 0 || z < 0) ? MKey{~0ULL, ~0u, 0}
+                                       : make_key((unsigned int)x, (unsigned int)y, (unsigned int)z, d - 1);
   }
+}
+
+__global__ void nbr_parents(const MKey* __restrict__ S, long n, int d, int periodic, MKey* __restrict__ out) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  MKey c[8];
+  parent_candidates(S[i], d, periodic, c);
+  for (int k = 0; k < 8; ++k) out[i * 8 + k] = c[k];
 }
 
 __global__ void split_keys(const MKey* __restrict__ k, long n, unsigned long long* __restrict__ hi,
@@ -243,49 +249,78 @@ __global__ void compact_keys(const unsigned long long* __restrict__ hi, const un
   out[offs[i]] = k;
 }
 
-// ------------------------------------------------------------------ final tree
-__global__ void children_of(const MKey* __restrict__ S, long n, int d, MKey* __restrict__ out) {
+// The balance candidates of level d - 1 <= 21 as the hi words of their keys
+// (see sort_unique): R of that level, then the nbr_parents of S, where a
+// neighbour outside the box repeats the node's own parent.
+__global__ void candidate_hi(const MKey* __restrict__ R, long nR, const MKey* __restrict__ S, long nS, int d,
+                             int periodic, unsigned long long* __restrict__ hi) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  unsigned int X, Y, Z, dd;
-  decode_key(S[i], X, Y, Z, dd);
-  const unsigned int w = kTwo30 >> (d + 1);
-  for (int c = 0; c < 8; ++c)
-    out[i * 8 + c] = make_key(X + ((c & 1) ? w : 0), Y + ((c & 2) ? w : 0), Z + ((c & 4) ? w : 0), d + 1);
-}
-
-__global__ void member_flags(const MKey* __restrict__ keys, long n, const MKey* __restrict__ S, long nS,
-                             int* __restrict__ internal) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int f = 0;
-  if (nS > 0) {
-    const long p = lower_bound_key(S, nS, keys[i]);
-    f = (p < nS && key_eq(S[p], keys[i])) ? 1 : 0;
+  if (i < nR) {
+    hi[i] = R[i].hi;
+    return;
   }
-  internal[i] = f;
+  const long j = i - nR;
+  if (j >= nS) return;
+  MKey c[8];
+  parent_candidates(S[j], d, periodic, c);
+  for (int k = 0; k < 8; ++k) hi[nR + j * 8 + k] = c[k].hi == ~0ULL ? c[0].hi : c[k].hi;
 }
 
-// Links of one level.  `cap` is the level's internal-node count known on the
-// host (the size of the next level / 8 and of this level's int_idx segment);
-// the scan's own total is checked against it only after the build's final
-// synchronisation, so a rank k >= cap is skipped here instead of written out
-// of bounds (the host check then reports the mismatch).
-__global__ void level_links(const int* __restrict__ internal, const int* __restrict__ offs, long n, long base,
-                            long next_base, long int_base, long cap, unsigned char* __restrict__ leaf,
-                            int* __restrict__ child0, int* __restrict__ parent, int* __restrict__ int_idx) {
+__global__ void keys_from_hi(const unsigned long long* __restrict__ hi, long n, unsigned int lo,
+                             MKey* __restrict__ out) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const long g = base + i;
-  if (internal[i] && offs[i] < cap) {
-    const long k = offs[i];
-    leaf[g] = 0;
-    child0[g] = (int)(next_base + 8 * k);
-    int_idx[int_base + k] = (int)g;
-    for (int c = 0; c < 8; ++c) parent[next_base + 8 * k + c] = (int)g;
-  } else {
-    leaf[g] = 1;
-    child0[g] = -1;
+  if (i < n) out[i] = MKey{hi[i], lo, 0};
+}
+
+// ------------------------------------------------------------------ final tree
+// Levels of the final tree: S[d] the sorted keys of the internal nodes of
+// level d (n[d] of them), whose children, eight in a row, are level d + 1
+// (nodes off[d + 1] ..); ioff[d] numbers the internal nodes through all levels.
+struct LevelTab {
+  const MKey* S[kMaxDepth];
+  long n[kMaxDepth + 1], off[kMaxDepth + 2], ioff[kMaxDepth + 1];
+  int depth;  // levels with internal nodes
+};
+
+// One thread per internal node of any level: its place in its level is 8 times
+// its parent's rank (a search of the level above) plus its octant; it writes
+// its own links and its children's keys and parents.  Leaves keep what the
+// arrays are preset to (leaf 1, child0 -1, parent 0).  A parent missing from
+// the level above (the set is not closed) is reported in *bad and linked to
+// the root, so that nothing is read or written out of range.
+__global__ void link_nodes(LevelTab lt, long n_int, MKey* __restrict__ keys, unsigned char* __restrict__ leaf,
+                           int* __restrict__ child0, int* __restrict__ parent, int* __restrict__ int_idx,
+                           int* __restrict__ bad) {
+  const long j = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (j == 0) {
+    keys[0] = make_key(0, 0, 0, 0);
+    parent[0] = -1;
+  }
+  if (j >= n_int) return;
+  int d = 0;
+  while (d + 1 < lt.depth && j >= lt.ioff[d + 1]) ++d;
+  const long k = j - lt.ioff[d];
+  unsigned int q[3], dd;
+  const MKey key = lt.S[d][k];
+  decode_key(key, q[0], q[1], q[2], dd);
+  long g = 0;
+  if (d > 0) {
+    const unsigned int w = kTwo30 >> d, m = ~(2 * w - 1);
+    const MKey pk = make_key(q[0] & m, q[1] & m, q[2] & m, d - 1);
+    const long r = lower_bound_key(lt.S[d - 1], lt.n[d - 1], pk);
+    if (r < lt.n[d - 1] && key_eq(lt.S[d - 1][r], pk))
+      g = lt.off[d] + 8 * r + ((q[0] & w ? 1 : 0) | (q[1] & w ? 2 : 0) | (q[2] & w ? 4 : 0));
+    else
+      *bad = 1;
+  }
+  const long c0 = lt.off[d + 1] + 8 * k;
+  leaf[g] = 0;
+  child0[g] = (int)c0;
+  int_idx[j] = (int)g;
+  const unsigned int w = kTwo30 >> (d + 1);
+  for (int c = 0; c < 8; ++c) {
+    keys[c0 + c] = make_key(q[0] + ((c & 1) ? w : 0), q[1] + ((c & 2) ? w : 0), q[2] + ((c & 4) ? w : 0), d + 1);
+    parent[c0 + c] = (int)g;
   }
 }
 
@@ -353,15 +388,14 @@ template <class Real>
 __global__ void localize(const int* __restrict__ leaves, long n_leaves, const MKey* __restrict__ keys,
                          const int* __restrict__ lo, const int* __restrict__ hi, const double* __restrict__ coord,
                          Real* __restrict__ x, Real* __restrict__ y, Real* __restrict__ z, int* __restrict__ pt_leaf) {
-  const long li = blockIdx.x;
+  const long li = blockIdx.x * (long)(blockDim.x / 32) + threadIdx.x / 32;  // a warp per leaf
   if (li >= n_leaves) return;
   const int node = leaves[li];
-  if (node < 0) return;  // slot left unfilled by a count mismatch (reported by the host)
   unsigned int X, Y, Z, d;
   decode_key(keys[node], X, Y, Z, d);
   const double h = 1.0 / (double)(1u << d);
   const double c[3] = {X * (1.0 / kTwo30) + 0.5 * h, Y * (1.0 / kTwo30) + 0.5 * h, Z * (1.0 / kTwo30) + 0.5 * h};
-  for (int p = lo[node] + threadIdx.x; p < hi[node]; p += blockDim.x) {
+  for (int p = lo[node] + threadIdx.x % 32; p < hi[node]; p += 32) {
     x[p] = (Real)(coord[p * 3 + 0] - c[0]);
     y[p] = (Real)(coord[p * 3 + 1] - c[1]);
     z[p] = (Real)(coord[p * 3 + 2] - c[2]);
@@ -401,6 +435,19 @@ __device__ __forceinline__ unsigned char image_code(const MKey* keys, long v, in
   return (unsigned char)code;
 }
 
+// Memberships (0 or 1) and list lengths of a node, summed together.
+enum { kSleaf, kTleaf, kVsrc, kP2P, kX, kW, kXtrg, kVtrg, kLeaf, kNodeCounts };
+struct NodeCounts {
+  int v[kNodeCounts];
+};
+struct SumCounts {
+  __host__ __device__ NodeCounts operator()(const NodeCounts& a, const NodeCounts& b) const {
+    NodeCounts c;
+    for (int i = 0; i < kNodeCounts; ++i) c.v[i] = a.v[i] + b.v[i];
+    return c;
+  }
+};
+
 // One pass per target node (n_trg > 0); `mode` 0 counts, 1 fills.
 // Relative coordinates follow InteracList::BuildList (interac_list.txx:98-279).
 // With image arrays (periodic boundaries) every entry also gets the image
@@ -409,9 +456,8 @@ __device__ __forceinline__ unsigned char image_code(const MKey* keys, long v, in
 __global__ void build_lists(long n_nodes, const unsigned char* __restrict__ leaf, const int* __restrict__ parent,
                             const int* __restrict__ child0, const int* __restrict__ coll, const int* __restrict__ slo,
                             const int* __restrict__ shi, const int* __restrict__ tlo, const int* __restrict__ thi,
-                            long nsrf, int sw, int mode, int* __restrict__ p_cnt, int* __restrict__ x_cnt,
-                            int* __restrict__ w_cnt,
-                            int* __restrict__ v_cnt, const int* __restrict__ p_off, const int* __restrict__ x_off,
+                            long nsrf, int sw, int mode, NodeCounts* __restrict__ counts,
+                            const int* __restrict__ p_off, const int* __restrict__ x_off,
                             const int* __restrict__ w_off, int* __restrict__ p_list, int* __restrict__ x_list,
                             int* __restrict__ w_list, const MKey* __restrict__ keys, unsigned char* __restrict__ p_img,
                             unsigned char* __restrict__ x_img, unsigned char* __restrict__ w_img) {
@@ -500,25 +546,68 @@ __global__ void build_lists(long n_nodes, const unsigned char* __restrict__ leaf
 #undef ADD
   }
   if (!mode) {
-    p_cnt[t] = np;
-    x_cnt[t] = nx;
-    w_cnt[t] = nw;
-    v_cnt[t] = nv;
+    const bool lf = leaf[t], src = shi[t] > slo[t];
+    NodeCounts c;
+    c.v[kSleaf] = lf && src;
+    c.v[kTleaf] = lf && nt > 0;
+    c.v[kVsrc] = !lf && src;
+    c.v[kP2P] = np;
+    c.v[kX] = nx;
+    c.v[kW] = nw;
+    c.v[kXtrg] = nx > 0;
+    c.v[kVtrg] = nv > 0;
+    c.v[kLeaf] = lf;
+    counts[t] = c;
+  }
+}
+
+struct NodeLists {
+  int *sleaf, *tleaf, *vsrc, *xtrg, *vtrg;
+};
+
+// Places every node in the lists it belongs to, from the prefix sums of the
+// counts; ranks >= cap (the capacity of the lists) are skipped.  The last node
+// closes the CSR offsets and writes the totals to the pinned slots.
+__global__ void scatter_lists(long n, long cap, const NodeCounts* __restrict__ counts,
+                              const NodeCounts* __restrict__ offs, NodeLists l, int* __restrict__ node2vsrc,
+                              int* __restrict__ po, int* __restrict__ xo, int* __restrict__ wo,
+                              int* __restrict__ totals) {
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const NodeCounts c = counts[t], o = offs[t];
+  if (c.v[kSleaf] && o.v[kSleaf] < cap) l.sleaf[o.v[kSleaf]] = (int)t;
+  if (c.v[kTleaf] && o.v[kTleaf] < cap) l.tleaf[o.v[kTleaf]] = (int)t;
+  const bool vs = c.v[kVsrc] && o.v[kVsrc] < cap;
+  if (vs) l.vsrc[o.v[kVsrc]] = (int)t;
+  node2vsrc[t] = vs ? o.v[kVsrc] : -1;
+  if (c.v[kXtrg] && o.v[kXtrg] < cap) l.xtrg[o.v[kXtrg]] = (int)t;
+  if (c.v[kVtrg] && o.v[kVtrg] < cap) l.vtrg[o.v[kVtrg]] = (int)t;
+  po[t] = o.v[kP2P];
+  xo[t] = o.v[kX];
+  wo[t] = o.v[kW];
+  if (t == n - 1) {
+    const NodeCounts sum = SumCounts()(o, c);
+    po[n] = sum.v[kP2P];
+    xo[n] = sum.v[kX];
+    wo[n] = sum.v[kW];
+    for (int i = 0; i < kNodeCounts; ++i) totals[i] = sum.v[i];
   }
 }
 
 // V-list targets are ordered by their pattern of occupied offsets within
 // windows of kVsortWindow consecutive (Morton-ordered) targets: bit o of the
 // pattern is set when the target has a source parent at colleague offset o
-// (the offsets of fill_vtab).  key[i] = window << 26 | pattern.
+// (the offsets of vlist_order).  key[i] = window << 26 | pattern.
 #ifndef PVFMM_VSORT_WINDOW
 #define PVFMM_VSORT_WINDOW 2048
 #endif
 constexpr long kVsortWindow = PVFMM_VSORT_WINDOW;
 __global__ void vlist_keys(const int* __restrict__ vtrg, long n_vtrg, const int* __restrict__ coll,
-                           const int* __restrict__ node2vsrc, unsigned long long* __restrict__ key) {
+                           const int* __restrict__ node2vsrc, unsigned long long* __restrict__ key,
+                           int* __restrict__ rank) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n_vtrg) return;
+  rank[i] = (int)i;
   const long t = vtrg[i];
   unsigned m = 0;
   for (int ci = 0, o = 0; ci < 27; ++ci) {
@@ -530,50 +619,25 @@ __global__ void vlist_keys(const int* __restrict__ vtrg, long n_vtrg, const int*
   key[i] = (unsigned long long)(i / kVsortWindow) << 26 | m;
 }
 // Pattern order from the sorted Morton ranks: position p takes the node of
-// rank rank_sorted[p]; vmorton[rank] = p.
-__global__ void vlist_reorder(const int* __restrict__ vtrg_morton, const int* __restrict__ rank_sorted, long n,
-                              int* __restrict__ vtrg_sorted, int* __restrict__ vmorton) {
+// rank rank_sorted[p], with its pattern and its row of source parents per
+// offset (offset-major: coalesced); vmorton[rank] = p.
+__global__ void vlist_order(const int* __restrict__ vtrg_morton, const int* __restrict__ rank_sorted,
+                            const unsigned long long* __restrict__ key_sorted, long n, const int* __restrict__ coll,
+                            const int* __restrict__ node2vsrc, int* __restrict__ vtrg, int* __restrict__ vmorton,
+                            unsigned* __restrict__ mask, int* __restrict__ vtab) {
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (p >= n) return;
   const int r = rank_sorted[p];
-  vtrg_sorted[p] = vtrg_morton[r];
+  const long t = vtrg_morton[r];
+  vtrg[p] = (int)t;
   vmorton[r] = (int)p;
-}
-
-__global__ void vlist_patterns(const unsigned long long* __restrict__ key, long n, unsigned* __restrict__ mask) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i < n) mask[i] = (unsigned)(key[i] & ((1u << 26) - 1));
-}
-
-__global__ void fill_vtab(const int* __restrict__ vtrg, long n_vtrg, const int* __restrict__ coll,
-                          const int* __restrict__ node2vsrc, int* __restrict__ vtab) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n_vtrg) return;
-  const long t = vtrg[i];
+  mask[p] = (unsigned)(key_sorted[p] & ((1u << 26) - 1));
   for (int ci = 0, o = 0; ci < 27; ++ci) {
     if (ci == 13) continue;
     const int c = coll[t * 27 + ci];
-    vtab[(long)o * n_vtrg + i] = (c >= 0) ? node2vsrc[c] : -1;  // offset-major: coalesced per offset
+    vtab[(long)o * n + p] = c >= 0 ? node2vsrc[c] : -1;
     ++o;
   }
-}
-
-template <class Pred>
-__global__ void flag_nodes(long n, Pred pred, int* __restrict__ flag) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i < n) flag[i] = pred(i) ? 1 : 0;
-}
-
-// out[offs[i]] = i for flagged i; ranks >= cap (the capacity of out) are
-// skipped, so a count that disagrees with the host's expectation (checked
-// after the build's final synchronisation) never writes out of bounds.
-__global__ void compact_index(const int* __restrict__ flag, const int* __restrict__ offs, long n, long cap,
-                              int* __restrict__ out, int* __restrict__ map) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const bool f = flag[i] && offs[i] < cap;
-  if (f) out[offs[i]] = (int)i;
-  if (map) map[i] = f ? offs[i] : -1;
 }
 
 __global__ void gather_u32(const unsigned int* __restrict__ in, const int* __restrict__ perm, long n,
@@ -587,52 +651,30 @@ __global__ void iota_kernel(int* __restrict__ a, long n) {
   if (i < n) a[i] = (int)i;
 }
 
-// Pinned host slots of a tree build (ctx.chk): the deferred counts, two
-// slots for the totals read back at once, and 12 doubles of bounding boxes.
-constexpr int kChkLists = 40, kChkLeaves = 48, kChkScan = 60, kChkSlots = 64;
+// Pinned host slots of a tree build (ctx.chk): the list totals, the error word
+// of link_nodes, the last scan's total, and 12 doubles of bounding boxes.
+constexpr int kChkLists = 0, kChkLinks = 16, kChkScan = 17, kChkSlots = 32;
 constexpr size_t kChkBytes = kChkSlots * sizeof(int) + 12 * sizeof(double);
 inline double* chk_bbox(Context& ctx) { return reinterpret_cast<double*>(ctx.chk + kChkSlots); }
 
-// Exclusive prefix sum of n ints; returns the total (synchronous read through
-// pinned slots).
+// The total out[n-1] + in[n-1] of an exclusive scan, into a pinned slot.
+__global__ void scan_total(const int* __restrict__ in, const int* __restrict__ out, long n, int* __restrict__ slot) {
+  *slot = out[n - 1] + in[n - 1];
+}
+
+// Exclusive prefix sum of n ints; returns the total (read through a pinned
+// slot after a synchronisation).
 long exclusive_scan(Context& ctx, const int* in, int* out, long n) {
   if (n <= 0) return 0;
   size_t bytes = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int)n, ctx.stream);
   void* tmp = ctx.scratch2.ensure(bytes);
   cub::DeviceScan::ExclusiveSum(tmp, bytes, in, out, (int)n, ctx.stream);
-  int* h = ctx.chk + kChkScan;
-  PVFMM_CUDA_CHECK(cudaMemcpyAsync(&h[0], out + n - 1, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
-  PVFMM_CUDA_CHECK(cudaMemcpyAsync(&h[1], in + n - 1, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
-  PVFMM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
-  return (long)h[0] + h[1];
-}
-
-// Pinned count slots of a tree build: [0, kMaxDepth] internal nodes per level,
-// then the compacted list sizes and the leaf count.
-static_assert(kMaxDepth < kChkLists, "per-level slots overlap the list slots");
-
-// Exclusive prefix sum of n ints without reading the total back; the total
-// (out[n-1] + in[n-1]) is copied into the pinned slot *slot (valid after the
-// stream's next synchronisation) and, with `close`, also stored as out[n].
-__global__ void scan_total(const int* __restrict__ in, int* __restrict__ out, long n, int* __restrict__ slot,
-                           bool close) {
-  const int t = out[n - 1] + in[n - 1];
-  *slot = t;
-  if (close) out[n] = t;
-}
-
-void exclusive_scan_deferred(Context& ctx, const int* in, int* out, long n, int* slot, bool close = false) {
-  if (n <= 0) {
-    *slot = 0;
-    return;
-  }
-  size_t bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int)n, ctx.stream);
-  void* tmp = ctx.scratch2.ensure(bytes);
-  cub::DeviceScan::ExclusiveSum(tmp, bytes, in, out, (int)n, ctx.stream);
+  int* slot = ctx.chk + kChkScan;
   ++ctx.n_launch;
-  scan_total<<<1, 1, 0, ctx.stream>>>(in, out, n, slot, close);
+  scan_total<<<1, 1, 0, ctx.stream>>>(in, out, n, slot);
+  PVFMM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
+  return *(volatile int*)slot;
 }
 
 // Stable sort of 96-bit keys (hi, lo): by lo, then stably by hi.  On return
@@ -658,56 +700,49 @@ void sort_hilo(Context& ctx, long n, const unsigned long long* hi, const unsigne
   gather_u32<<<ceil_div(n, kThreads), kThreads, 0, s>>>(lo, perm, n, ls);
 }
 
-__global__ void unique_flags_hi(const unsigned long long* __restrict__ hi, long n, int* __restrict__ flag) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  flag[i] = (hi[i] != ~0ULL && (i == 0 || hi[i] != hi[i - 1])) ? 1 : 0;
+// The sorted, unique keys of the level's internal nodes after balance: R (the
+// refined ones, nR) with the neighbours' parents of S, the balanced level d
+// below (nS nodes); returns their count.  A node of depth L = d - 1 <= 21 has
+// zero coordinate bits below 30 - L, so its key is hi (top 3L bits of the
+// 63-bit interleave) with lo = L: one keys-only radix sort over those bits
+// orders them.
+long balance_level(Context& ctx, const MKey* R, long nR, const MKey* S, long nS, int d, DevBuf& out) {
+  auto& s = ctx.stream;
+  const long n = nR + 8 * nS;
+  const int depth = d - 1;
+  unsigned long long* h = ctx.t[10].as<unsigned long long>(n);
+  unsigned long long* hs = ctx.t[13].as<unsigned long long>(n);
+  ++ctx.n_launch;
+  candidate_hi<<<ceil_div(nR + nS, kThreads), kThreads, 0, s>>>(R, nR, S, nS, d, ctx.periodic ? ctx.periodic_axes : 0,
+                                                               h);
+  const int begin_bit = 3 * (21 - depth);
+  size_t b1 = 0, b2 = 0;
+  int* slot = ctx.chk + kChkScan;
+  cub::DeviceRadixSort::SortKeys(nullptr, b1, h, hs, (int)n, begin_bit, 63, s);
+  cub::DeviceSelect::Unique(nullptr, b2, hs, h, slot, (int)n, s);
+  void* tmp = ctx.scratch.ensure(std::max(b1, b2));
+  // (a root-only level has no key bits: every candidate is the root)
+  const unsigned long long* sorted = h;
+  unsigned long long* uniq = hs;
+  if (begin_bit < 63) {
+    cub::DeviceRadixSort::SortKeys(tmp, b1, h, hs, (int)n, begin_bit, 63, s);
+    sorted = hs;
+    uniq = h;
+  }
+  cub::DeviceSelect::Unique(tmp, b2, sorted, uniq, slot, (int)n, s);
+  PVFMM_CUDA_CHECK(cudaStreamSynchronize(s));
+  const long cnt = *(volatile int*)slot;
+  MKey* o = out.as<MKey>(std::max(cnt, 1L));
+  ++ctx.n_launch;
+  keys_from_hi<<<ceil_div(std::max(cnt, 1L), kThreads), kThreads, 0, s>>>(uniq, cnt, (unsigned int)depth, o);
+  return cnt;
 }
 
-__global__ void compact_keys_hi(const unsigned long long* __restrict__ hi, const int* __restrict__ flag,
-                                const int* __restrict__ offs, long n, unsigned int lo, MKey* __restrict__ out) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n || !flag[i]) return;
-  MKey k;
-  k.hi = hi[i];
-  k.lo = lo;
-  k.pad = 0;
-  out[offs[i]] = k;
-}
-
-__global__ void key_hi(const MKey* __restrict__ k, long n, unsigned long long* __restrict__ hi) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i < n) hi[i] = k[i].hi;
-}
-
-// Sorts node keys of one depth and removes duplicates and sentinels; returns
-// the count.  A node of depth L <= 21 has zero coordinate bits below 30 - L,
-// so its key is hi (top 3L bits of the 63-bit interleave) with lo = L: one
-// keys-only radix sort over those bits (and bit 63, which only the sentinels
-// set) orders them.  Deeper levels use the full 96-bit sort.
-long sort_unique(Context& ctx, const MKey* in, long n, DevBuf& out, int depth) {
+// Sorts node keys (of levels deeper than 21: full 96-bit keys) and removes
+// duplicates and sentinels; returns the count.
+long sort_unique(Context& ctx, const MKey* in, long n, DevBuf& out) {
   auto& s = ctx.stream;
   if (n == 0) return 0;
-  if (depth <= 21) {
-    unsigned long long* h = ctx.t[10].as<unsigned long long>(n);
-    unsigned long long* hs = ctx.t[13].as<unsigned long long>(n);
-    ++ctx.n_launch;
-    key_hi<<<ceil_div(n, kThreads), kThreads, 0, s>>>(in, n, h);
-    const int begin_bit = 3 * (21 - depth);
-    size_t bytes = 0;
-    cub::DeviceRadixSort::SortKeys(nullptr, bytes, h, hs, (int)n, begin_bit, 64, s);
-    void* tmp = ctx.scratch.ensure(bytes);
-    cub::DeviceRadixSort::SortKeys(tmp, bytes, h, hs, (int)n, begin_bit, 64, s);
-    int* fl = ctx.t[19].as<int>(n);
-    int* of = ctx.t[20].as<int>(n);
-    ++ctx.n_launch;
-    unique_flags_hi<<<ceil_div(n, kThreads), kThreads, 0, s>>>(hs, n, fl);
-    const long cnt = exclusive_scan(ctx, fl, of, n);
-    MKey* o = out.as<MKey>(std::max(cnt, 1L));
-    ++ctx.n_launch;
-    compact_keys_hi<<<ceil_div(n, kThreads), kThreads, 0, s>>>(hs, fl, of, n, (unsigned int)depth, o);
-    return cnt;
-  }
   unsigned long long* h = ctx.t[10].as<unsigned long long>(n);
   unsigned int* l = ctx.t[11].as<unsigned int>(n);
   int* ix = ctx.t[12].as<int>(n);
@@ -894,15 +929,22 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
   //    targets for a unit-box tree (pt_coord = trg_coord, pvfmm.txx:238)
   const MKey* sk = T.src_counted ? T.src_key.get<MKey>() : nullptr;
   const MKey* tk = T.trg_key.get<MKey>();
-  std::vector<MKey> gk;
   const MKey* d_gk = tk;
   long n_gk = n_trg;
   if (!ctx.unit_box) {
-    gk = seed_grid_keys(ctx.max_pts, pos_float);
-    MKey* g = ctx.t[9].as<MKey>(gk.size());
-    PVFMM_CUDA_CHECK(cudaMemcpyAsync(g, gk.data(), gk.size() * sizeof(MKey), cudaMemcpyHostToDevice, s));
-    d_gk = g;
-    n_gk = (long)gk.size();
+    // the same for every tree of the context (max_pts and the coordinates'
+    // precision): uploaded once
+    if (ctx.n_seed == 0 || ctx.seed_float != pos_float) {
+      const std::vector<MKey> gk = seed_grid_keys(ctx.max_pts, pos_float);
+      ctx.n_seed = 0;
+      MKey* g = ctx.seed.as<MKey>(gk.size());
+      PVFMM_CUDA_CHECK(cudaMemcpyAsync(g, gk.data(), gk.size() * sizeof(MKey), cudaMemcpyHostToDevice, s));
+      PVFMM_CUDA_CHECK(cudaStreamSynchronize(s));  // gk goes out of scope
+      ctx.n_seed = (long)gk.size();
+      ctx.seed_float = pos_float;
+    }
+    d_gk = ctx.seed.get<MKey>();
+    n_gk = ctx.n_seed;
   }
   // 5. refinement, level by level
   std::vector<long> nR;
@@ -943,6 +985,11 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
                                      nR[dint] * sizeof(MKey), cudaMemcpyDeviceToDevice, s));
     nS[dint] = nR[dint];
     for (int d = dint; d >= 1; --d) {
+      if (d - 1 <= 21) {
+        nS[d - 1] = balance_level(ctx, ctx.lvlR[d - 1].get<MKey>(), nR[d - 1], ctx.lvlS[d].get<MKey>(), nS[d], d,
+                                  ctx.lvlS[d - 1]);
+        continue;
+      }
       const long nc = nR[d - 1] + 8 * nS[d];
       MKey* cand = ctx.t[9].as<MKey>(nc);
       PVFMM_CUDA_CHECK(cudaMemcpyAsync(cand, ctx.lvlR[d - 1].get<MKey>(), nR[d - 1] * sizeof(MKey),
@@ -951,7 +998,7 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
       nbr_parents<<<ceil_div(nS[d], kThreads), kThreads, 0, s>>>(ctx.lvlS[d].get<MKey>(), nS[d], d,
                                                                  ctx.periodic ? ctx.periodic_axes : 0,
                                                                  cand + nR[d - 1]);
-      nS[d - 1] = sort_unique(ctx, cand, nc, ctx.lvlS[d - 1], d - 1);
+      nS[d - 1] = sort_unique(ctx, cand, nc, ctx.lvlS[d - 1]);
     }
   }
   // 7. final node arrays
@@ -972,35 +1019,27 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
   for (int d = 0; d < D; ++d) n_int_total += nS[d];
   int* int_idx = T.int_idx.as<int>(std::max(n_int_total, 1L));
   T.int_off.assign(D + 1, 0);
-  {
-    MKey root = make_key(0, 0, 0, 0);
-    PVFMM_CUDA_CHECK(cudaMemcpyAsync(keys, &root, sizeof(MKey), cudaMemcpyHostToDevice, s));
-    const int minus1 = -1;
-    PVFMM_CUDA_CHECK(cudaMemcpyAsync(parent, &minus1, sizeof(int), cudaMemcpyHostToDevice, s));
-  }
+  LevelTab lt{};
+  lt.depth = D;
   long int_base = 0;
   for (int d = 0; d <= D; ++d) {
-    const long base = T.level_off[d], nl = T.level_off[d + 1] - base;
-    if (d > 0) ++ctx.n_launch;
-    if (d > 0) children_of<<<ceil_div(nS[d - 1], kThreads), kThreads, 0, s>>>(ctx.lvlS[d - 1].get<MKey>(), nS[d - 1],
-                                                                              d - 1, keys + base);
-    int* internal = ctx.t[3].as<int>(nl);
-    int* offs = ctx.t[23].as<int>(nl);
-    const long nSd = d < D ? nS[d] : 0;
-    ++ctx.n_launch;
-    member_flags<<<ceil_div(nl, kThreads), kThreads, 0, s>>>(keys + base, nl, d < D ? ctx.lvlS[d].get<MKey>() : nullptr,
-                                                             nSd, internal);
-    // the count is known (nSd); the scan's total is checked after the build's
-    // final synchronisation instead of waiting for it here
-    exclusive_scan_deferred(ctx, internal, offs, nl, ctx.chk + d);
-    const long nint = nSd;
+    const long nint = d < D ? nS[d] : 0;
     T.n_internal[d] = nint;
     T.int_off[d] = int_base;
-    ++ctx.n_launch;
-    level_links<<<ceil_div(nl, kThreads), kThreads, 0, s>>>(internal, offs, nl, base, T.level_off[d + 1], int_base,
-                                                            nSd, leaf, child0, parent, int_idx);
+    if (d < D) lt.S[d] = ctx.lvlS[d].get<MKey>();
+    lt.n[d] = nint;
+    lt.off[d] = T.level_off[d];
+    lt.ioff[d] = int_base;
     int_base += nint;
   }
+  lt.off[D + 1] = N;
+  ctx.chk[kChkLinks] = 0;  // (nothing in flight writes it)
+  PVFMM_CUDA_CHECK(cudaMemsetAsync(leaf, 1, N, s));
+  PVFMM_CUDA_CHECK(cudaMemsetAsync(child0, 0xff, N * sizeof(int), s));
+  PVFMM_CUDA_CHECK(cudaMemsetAsync(parent, 0, N * sizeof(int), s));
+  ++ctx.n_launch;
+  link_nodes<<<ceil_div(std::max(n_int_total, 1L), 128), 128, 0, s>>>(lt, n_int_total, keys, leaf, child0, parent,
+                                                                       int_idx, ctx.chk + kChkLinks);
   // 8. point ranges and colleagues
   int* slo = T.src_lo.as<int>(N);
   int* shi = T.src_hi.as<int>(N);
@@ -1015,51 +1054,43 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
     colleagues_kernel<<<ceil_div(nl, kThreads), kThreads, 0, s>>>(base, nl, parent, child0,
                                                                    ctx.periodic ? ctx.periodic_axes : 0, coll);
   }
-  // 9. compact node lists.  The compacted lists are sized for all N nodes so
-  //    that the eight counts are read back together at one synchronisation.
+  // 9. compact node lists.  Every node's memberships and list lengths are one
+  //    record of counts (NodeCounts), prefix-summed together; the compacted
+  //    lists are sized for all N nodes, so that their counts are read back at
+  //    one synchronisation.
   {
-    int* flag = ctx.t[3].as<int>(N);
-    int* offs = ctx.t[23].as<int>(N);
-    int* cnt = ctx.chk + kChkLists;  // sleaf tleaf vsrc p2p x w xtrg vtrg
-    auto compact = [&](auto pred, DevBuf& out, int* map, int* slot) {
-      ++ctx.n_launch;
-      flag_nodes<<<ceil_div(N, kThreads), kThreads, 0, s>>>(N, pred, flag);
-      exclusive_scan_deferred(ctx, flag, offs, N, slot);
-      int* o = out.as<int>(N);
-      ++ctx.n_launch;
-      compact_index<<<ceil_div(N, kThreads), kThreads, 0, s>>>(flag, offs, N, N, o, map);
-    };
-    compact([=] __device__(long i) { return leaf[i] && shi[i] > slo[i]; }, T.sleaf, nullptr, cnt + 0);
-    compact([=] __device__(long i) { return leaf[i] && thi[i] > tlo[i]; }, T.tleaf, nullptr, cnt + 1);
-    int* n2v = T.node2vsrc.as<int>(N);
-    compact([=] __device__(long i) { return !leaf[i] && shi[i] > slo[i]; }, T.vsrc, n2v, cnt + 2);
-    // lists: count
-    int* pc = ctx.t[4].as<int>(N);
-    int* xc = ctx.t[5].as<int>(N);
-    int* wc = ctx.t[6].as<int>(N);
-    int* vc = ctx.t[0].as<int>(N);
+    NodeCounts* nc = ctx.t[4].as<NodeCounts>(N);
+    NodeCounts* no = ctx.t[5].as<NodeCounts>(N);
+    int* cnt = ctx.chk + kChkLists;
     const long nsrf = ctx.ns;
     ++ctx.n_launch;
     build_lists<<<ceil_div(N, 128), 128, 0, s>>>(N, leaf, parent, child0, coll, slo, shi, tlo, thi, nsrf,
-                                                 T.src_weight, 0, pc, xc, wc, vc, nullptr, nullptr, nullptr, nullptr,
-                                                 nullptr, nullptr, keys, nullptr, nullptr, nullptr);
+                                                 T.src_weight, 0, nc, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                                 nullptr, keys, nullptr, nullptr, nullptr);
+    size_t bytes = 0;
+    cub::DeviceScan::ExclusiveScan(nullptr, bytes, nc, no, SumCounts(), NodeCounts{}, (int)N, s);
+    void* stmp = ctx.scratch2.ensure(bytes);
+    cub::DeviceScan::ExclusiveScan(stmp, bytes, nc, no, SumCounts(), NodeCounts{}, (int)N, s);
     int* po = T.p_off.as<int>(N + 1);
     int* xo = T.x_off.as<int>(N + 1);
     int* wo = T.w_off.as<int>(N + 1);
-    exclusive_scan_deferred(ctx, pc, po, N, cnt + 3, true);
-    exclusive_scan_deferred(ctx, xc, xo, N, cnt + 4, true);
-    exclusive_scan_deferred(ctx, wc, wo, N, cnt + 5, true);
-    compact([=] __device__(long i) { return xc[i] > 0; }, T.xtrg, nullptr, cnt + 6);
-    compact([=] __device__(long i) { return vc[i] > 0; }, T.vtrg, nullptr, cnt + 7);
+    int* n2v = T.node2vsrc.as<int>(N);
+    int* vtrg_morton = ctx.t[0].as<int>(N);
+    ++ctx.n_launch;
+    scatter_lists<<<ceil_div(N, kThreads), kThreads, 0, s>>>(
+        N, N, nc, no, NodeLists{T.sleaf.as<int>(N), T.tleaf.as<int>(N), T.vsrc.as<int>(N), T.xtrg.as<int>(N), vtrg_morton},
+        n2v, po, xo, wo, cnt);
     PVFMM_CUDA_CHECK(cudaStreamSynchronize(s));
-    T.n_sleaf = cnt[0];
-    T.n_tleaf = cnt[1];
-    T.n_vsrc = cnt[2];
-    T.n_p2p = cnt[3];
-    T.n_x = cnt[4];
-    T.n_w = cnt[5];
-    T.n_xtrg = cnt[6];
-    T.n_vtrg = cnt[7];
+    T.n_sleaf = cnt[kSleaf];
+    T.n_tleaf = cnt[kTleaf];
+    T.n_vsrc = cnt[kVsrc];
+    T.n_p2p = cnt[kP2P];
+    T.n_x = cnt[kX];
+    T.n_w = cnt[kW];
+    T.n_xtrg = cnt[kXtrg];
+    T.n_vtrg = cnt[kVtrg];
+    if (cnt[kLeaf] != (int)(N - n_int_total) || ctx.chk[kChkLinks] != 0)
+      throw std::runtime_error("octree build: balanced internal set is not closed");
     int* pl = T.p_list.as<int>(std::max(T.n_p2p, 1L));
     int* xl = T.x_list.as<int>(std::max(T.n_x, 1L));
     int* wl = T.w_list.as<int>(std::max(T.n_w, 1L));
@@ -1068,7 +1099,7 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
     unsigned char* wim = ctx.periodic ? T.w_img.as<unsigned char>(std::max(T.n_w, 1L)) : nullptr;
     ++ctx.n_launch;
     build_lists<<<ceil_div(N, 128), 128, 0, s>>>(N, leaf, parent, child0, coll, slo, shi, tlo, thi, nsrf,
-                                                 T.src_weight, 1, nullptr, nullptr, nullptr, nullptr, po, xo, wo, pl,
+                                                 T.src_weight, 1, nullptr, po, xo, wo, pl,
                                                  xl, wl, keys, pim, xim, wim);
     int* vt = T.vtab.as<int>(std::max(T.n_vtrg, 1L) * 26);
     unsigned* vm = T.vmask.as<unsigned>(std::max(T.n_vtrg, 1L));
@@ -1084,13 +1115,10 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
       // ranges of positions too).
       unsigned long long* key = ctx.t[10].as<unsigned long long>(T.n_vtrg);
       unsigned long long* keys_sorted = ctx.t[13].as<unsigned long long>(T.n_vtrg);
-      int* vs = ctx.t[11].as<int>(T.n_vtrg);
       int* rank_in = ctx.t[12].as<int>(T.n_vtrg);
       int* rank_sorted = ctx.t[14].as<int>(T.n_vtrg);
       ++ctx.n_launch;
-      vlist_keys<<<ceil_div(T.n_vtrg, kThreads), kThreads, 0, s>>>(T.vtrg.get<int>(), T.n_vtrg, coll, n2v, key);
-      ++ctx.n_launch;
-      iota_kernel<<<ceil_div(T.n_vtrg, kThreads), kThreads, 0, s>>>(rank_in, T.n_vtrg);
+      vlist_keys<<<ceil_div(T.n_vtrg, kThreads), kThreads, 0, s>>>(vtrg_morton, T.n_vtrg, coll, n2v, key, rank_in);
       int end_bit = 27;
       while (end_bit < 64 && ((T.n_vtrg - 1) / kVsortWindow) >> (end_bit - 26)) ++end_bit;
       size_t bytes = 0;
@@ -1101,31 +1129,13 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
                                       s);
       int* vmorton = T.vmorton.as<int>(T.n_vtrg);
       ++ctx.n_launch;
-      vlist_reorder<<<ceil_div(T.n_vtrg, kThreads), kThreads, 0, s>>>(T.vtrg.get<int>(), rank_sorted, T.n_vtrg, vs,
-                                                                      vmorton);
-      PVFMM_CUDA_CHECK(cudaMemcpyAsync(T.vtrg.get<int>(), vs, T.n_vtrg * sizeof(int), cudaMemcpyDeviceToDevice, s));
+      vlist_order<<<ceil_div(T.n_vtrg, kThreads), kThreads, 0, s>>>(vtrg_morton, rank_sorted, keys_sorted, T.n_vtrg, coll,
+                                                                    n2v, T.vtrg.as<int>(N), vmorton, vm, vt);
       T.vtiles_valid = false;
-      ++ctx.n_launch;
-      vlist_patterns<<<ceil_div(T.n_vtrg, kThreads), kThreads, 0, s>>>(keys_sorted, T.n_vtrg, vm);
-      ++ctx.n_launch;
-      fill_vtab<<<ceil_div(T.n_vtrg, kThreads), kThreads, 0, s>>>(T.vtrg.get<int>(), T.n_vtrg, coll, n2v, vt);
     }
   }
-  // 10. point -> leaf and local coordinates
+  // 10. point -> leaf and local coordinates, over the leaves with points
   {
-    const long n_leaves_all = N - n_int_total;
-    int* flag = ctx.t[3].as<int>(N);
-    int* offs = ctx.t[23].as<int>(N);
-    ++ctx.n_launch;
-    flag_nodes<<<ceil_div(N, kThreads), kThreads, 0, s>>>(N, [=] __device__(long i) { return leaf[i] != 0; }, flag);
-    // the leaf count is known; the scan's total is checked at the end
-    exclusive_scan_deferred(ctx, flag, offs, N, ctx.chk + kChkLeaves);
-    const long nl = n_leaves_all;
-    int* leaves = ctx.t[0].as<int>(std::max(nl, 1L));
-    // -1 marks a slot that no leaf filled (a count mismatch, reported below)
-    PVFMM_CUDA_CHECK(cudaMemsetAsync(leaves, 0xff, std::max(nl, 1L) * sizeof(int), s));
-    ++ctx.n_launch;
-    compact_index<<<ceil_div(N, kThreads), kThreads, 0, s>>>(flag, offs, N, nl, leaves, nullptr);
     double* sx = T.sx.as<double>(std::max(T.n_src, 1L));
     double* sy = T.sy.as<double>(std::max(T.n_src, 1L));
     double* sz = T.sz.as<double>(std::max(T.n_src, 1L));
@@ -1134,80 +1144,117 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
     double* tz = T.tz.as<double>(std::max(T.n_trg, 1L));
     int* sl = T.src_leaf.as<int>(std::max(T.n_src, 1L));
     int* tl = T.trg_leaf.as<int>(std::max(T.n_trg, 1L));
-    if (nl > 0) {
-      // source coordinates are localized even when sl_den is NULL (unused then)
+    if (T.n_sleaf > 0) {
       ++ctx.n_launch;
-      localize<double><<<nl, 128, 0, s>>>(leaves, nl, keys, slo, shi, coords_s.get<double>(), sx, sy, sz, sl);
+      localize<double><<<ceil_div(T.n_sleaf, 4), 128, 0, s>>>(T.sleaf.get<int>(), T.n_sleaf, keys, slo, shi,
+                                                             coords_s.get<double>(), sx, sy, sz, sl);
+    }
+    if (T.n_tleaf > 0) {
       ++ctx.n_launch;
-      localize<double><<<nl, 128, 0, s>>>(leaves, nl, keys, tlo, thi, coords_t.get<double>(), tx, ty, tz, tl);
+      localize<double><<<ceil_div(T.n_tleaf, 4), 128, 0, s>>>(T.tleaf.get<int>(), T.n_tleaf, keys, tlo, thi,
+                                                             coords_t.get<double>(), tx, ty, tz, tl);
     }
   }
-  PVFMM_CUDA_CHECK(cudaStreamSynchronize(s));
   PVFMM_CUDA_CHECK(cudaGetLastError());
-  for (int d = 0; d <= D; ++d)
-    if (ctx.chk[d] != (int)T.n_internal[d]) throw std::runtime_error("octree build: balanced internal set is not closed");
-  if (ctx.chk[kChkLeaves] != (int)(N - n_int_total)) throw std::runtime_error("octree build: leaf count mismatch");
-  T.valid = true;
+  T.valid = true;  // the evaluation is queued behind the last kernels
 }
 
 }  // namespace pvfmm_b200
 
-// Self-check of the bounded writes of the tree build's deferred count check
-// (internal entry point, used by the GPU tests; no counterpart in the
-// reference).  Runs compact_index and level_links with `n` flagged entries
-// against capacities of `cap` < n, in buffers followed by a guard band, and
-// checks that the ranks below cap are written and nothing at or beyond it.
-// Returns 0 when the bounds hold, 1 otherwise (message in PVFMMGetLastError).
+// Self-check of the bounded writes of the tree build (internal entry point,
+// used by the GPU tests; no counterpart in the reference).  Runs scatter_lists
+// with `n` nodes in every list against a capacity of `cap` < n, and link_nodes
+// on a set that is not closed, in buffers followed by a guard band, and checks
+// that what is in range is written and nothing beyond it.  Returns 0 when the
+// bounds hold, 1 otherwise (message in PVFMMGetLastError).
 extern "C" int PVFMMB200CheckBoundedWrites(long n, long cap) {
   using namespace pvfmm_b200;
   constexpr long kGuard = 64;
-  int* buf = nullptr;
-  unsigned char* lf = nullptr;
+  void* buf = nullptr;
   try {
     if (n <= 0 || cap < 0 || cap > n || n > (1L << 24)) throw std::runtime_error("bad sizes");
-    // flag[n] = 1, offs[n] = iota, out[cap + guard], child0/parent/int_idx sized for cap internal nodes
-    const long n_out = cap + kGuard, n_par = 8 * cap + kGuard;
-    const long total = 2 * n + n_out + n + n_par + n_out;
-    PVFMM_CUDA_CHECK(cudaMalloc((void**)&buf, total * sizeof(int)));
-    PVFMM_CUDA_CHECK(cudaMalloc((void**)&lf, n));
-    int* flag = buf;
-    int* offs = flag + n;
-    int* out = offs + n;
-    int* child0 = out + n_out;
-    int* parent = child0 + n;
-    int* int_idx = parent + n_par;
-    std::vector<int> h(total, -7);
-    for (long i = 0; i < n; ++i) {
-      h[i] = 1;
-      h[n + i] = (int)i;
-    }
-    PVFMM_CUDA_CHECK(cudaMemcpy(buf, h.data(), total * sizeof(int), cudaMemcpyHostToDevice));
-    compact_index<<<ceil_div(n, kThreads), kThreads>>>(flag, offs, n, cap, out, nullptr);
-    // one level of n nodes at base 0, its children at next_base = n
-    level_links<<<ceil_div(n, kThreads), kThreads>>>(flag, offs, n, 0, 0, 0, cap, lf, child0, parent, int_idx);
+    // records, then 5 lists of cap, node2vsrc (n), 3 offset arrays (n + 1) and
+    // the totals, each followed by a guard band
+    const long n_list = cap + kGuard, n_map = n + 1 + kGuard;
+    const long n_int = 5 * n_list + 4 * n_map + kNodeCounts + kGuard;
+    const size_t rec = (size_t)2 * n * sizeof(NodeCounts);
+    PVFMM_CUDA_CHECK(cudaMalloc(&buf, rec + n_int * sizeof(int)));
+    NodeCounts* nc = (NodeCounts*)buf;
+    int* w = (int*)(nc + 2 * n);
+    std::vector<NodeCounts> hr(2 * n);
+    for (long i = 0; i < n; ++i)
+      for (int k = 0; k < kNodeCounts; ++k) {
+        hr[i].v[k] = 1;
+        hr[n + i].v[k] = (int)i;
+      }
+    std::vector<int> h(n_int, -7);
+    PVFMM_CUDA_CHECK(cudaMemcpy(nc, hr.data(), rec, cudaMemcpyHostToDevice));
+    PVFMM_CUDA_CHECK(cudaMemcpy(w, h.data(), n_int * sizeof(int), cudaMemcpyHostToDevice));
+    int* map = w + 5 * n_list;
+    scatter_lists<<<ceil_div(n, kThreads), kThreads>>>(
+        n, cap, nc, nc + n, NodeLists{w, w + n_list, w + 2 * n_list, w + 3 * n_list, w + 4 * n_list}, map, map + n_map,
+        map + 2 * n_map, map + 3 * n_map, map + 4 * n_map);
     PVFMM_CUDA_CHECK(cudaGetLastError());
-    PVFMM_CUDA_CHECK(cudaMemcpy(h.data(), buf, total * sizeof(int), cudaMemcpyDeviceToHost));
+    PVFMM_CUDA_CHECK(cudaMemcpy(h.data(), w, n_int * sizeof(int), cudaMemcpyDeviceToHost));
+    for (int l = 0; l < 5; ++l)
+      for (long k = 0; k < n_list; ++k)
+        if (h[l * n_list + k] != (k < cap ? (int)k : -7))
+          throw std::runtime_error("scatter_lists wrote rank " + std::to_string(k) + " wrongly");
+    for (int l = 0; l < 4; ++l)
+      for (long k = 0; k < n_map; ++k) {
+        const int want = l == 0 ? (k < cap ? (int)k : k < n ? -1 : -7) : (k <= n ? (int)k : -7);
+        if (h[5 * n_list + l * n_map + k] != want)
+          throw std::runtime_error("scatter_lists wrote entry " + std::to_string(k) + " of an offset array wrongly");
+      }
+    for (long k = 0; k < kNodeCounts + kGuard; ++k)
+      if (h[5 * n_list + 4 * n_map + k] != (k < kNodeCounts ? (int)n : -7))
+        throw std::runtime_error("scatter_lists wrote the totals wrongly");
     cudaFree(buf);
-    cudaFree(lf);
     buf = nullptr;
-    lf = nullptr;
-    const int* ho = h.data() + 2 * n;
-    const int* hp = ho + n_out + n;
-    const int* hi = hp + n_par;
-    for (long k = 0; k < n_out; ++k) {
-      const int want = k < cap ? (int)k : -7;
-      if (ho[k] != want) throw std::runtime_error("compact_index wrote rank " + std::to_string(k) + " wrongly");
-      if (hi[k] != want) throw std::runtime_error("level_links wrote int_idx rank " + std::to_string(k) + " wrongly");
+    // a root and, at level 2, n internal nodes whose parents are not in level
+    // 1 (one internal node, the last octant): 1 + 8 + 8 + 8 n tree nodes
+    const long N = 17 + 8 * n, NG = N + kGuard;
+    std::vector<MKey> S(n + 2);
+    S[0] = make_key(0, 0, 0, 0);
+    S[1] = make_key(kTwo30 / 2, kTwo30 / 2, kTwo30 / 2, 1);
+    for (long i = 0; i < n; ++i) S[2 + i] = make_key(0, 0, 0, 2);
+    const size_t bytes = (S.size() + NG) * sizeof(MKey) + (size_t)(2 * NG + n + 2 + kGuard + 1) * sizeof(int) + NG;
+    PVFMM_CUDA_CHECK(cudaMalloc(&buf, bytes));
+    PVFMM_CUDA_CHECK(cudaMemset(buf, 0, bytes));
+    MKey* dS = (MKey*)buf;
+    MKey* keys = dS + S.size();
+    int* child0 = (int*)(keys + NG);
+    int* parent = child0 + NG;
+    int* int_idx = parent + NG;
+    int* bad = int_idx + n + 2 + kGuard;
+    unsigned char* lf = (unsigned char*)(bad + 1);
+    PVFMM_CUDA_CHECK(cudaMemcpy(dS, S.data(), S.size() * sizeof(MKey), cudaMemcpyHostToDevice));
+    PVFMM_CUDA_CHECK(cudaMemset(child0, 0xff, 2 * NG * sizeof(int)));
+    LevelTab lt{};
+    lt.depth = 3;
+    const long cnts[3] = {1, 1, n};
+    lt.off[1] = 1;
+    for (int d = 0; d < 3; ++d) {
+      lt.S[d] = dS + lt.ioff[d];
+      lt.n[d] = cnts[d];
+      lt.ioff[d + 1] = lt.ioff[d] + cnts[d];
+      lt.off[d + 2 > 3 ? 3 : d + 1] = d == 0 ? 1 : d == 1 ? 9 : 17;
     }
-    for (long k = 0; k < n_par; ++k) {
-      const int want = k < 8 * cap ? (int)(k / 8) : -7;
-      if (hp[k] != want) throw std::runtime_error("level_links wrote parent slot " + std::to_string(k) + " wrongly");
-    }
+    lt.off[3] = 17;
+    link_nodes<<<ceil_div(n + 2, 128), 128>>>(lt, n + 2, keys, lf, child0, parent, int_idx, bad);
+    PVFMM_CUDA_CHECK(cudaGetLastError());
+    std::vector<int> hc(2 * NG);
+    int hb = 0;
+    PVFMM_CUDA_CHECK(cudaMemcpy(hc.data(), child0, 2 * NG * sizeof(int), cudaMemcpyDeviceToHost));
+    PVFMM_CUDA_CHECK(cudaMemcpy(&hb, bad, sizeof(int), cudaMemcpyDeviceToHost));
+    if (hb != 1) throw std::runtime_error("link_nodes did not report the missing parents");
+    for (long k = N; k < NG; ++k)
+      if (hc[k] != -1 || hc[NG + k] != -1) throw std::runtime_error("link_nodes wrote out of range");
+    cudaFree(buf);
     set_last_error("");
     return 0;
   } catch (const std::exception& e) {
     if (buf) cudaFree(buf);
-    if (lf) cudaFree(lf);
     set_last_error(e.what());
     return 1;
   }
