@@ -17,9 +17,14 @@
 //
 // Tiling: a block computes a 128 x 64 tile of C with 8 warps (4 x 2), each
 // warp a 32 x 32 tile = 4 x 4 MMA tiles of 8 x 8, FP64 accumulators in
-// registers (each A and B fragment feeds four MMAs).
-// K advances in steps of 16; the A and B tiles of the next step are copied
-// into shared memory with 16-byte cp.async while the current step runs.
+// registers (each A and B fragment feeds four MMAs); few rows take 32 x 64
+// tiles (2 x 4 warps of 16 x 16).  Every sum runs over k in order, whatever
+// the tile, so the choice changes no value.
+// K advances in steps of 16; the A and B tiles of the next steps are copied
+// into shared memory with 16-byte cp.async behind the current step's first
+// MMAs, one barrier per step (4M clustered points, D2T products: 1.37 ms,
+// against 1.41 with a second barrier and the copies issued first, and 1.41
+// with three steps in shared memory).
 // Row lengths are even (ns = 6(m-1)^2+2), so every row of A, B and C starts
 // on a 16-byte boundary.
 #include <algorithm>
@@ -29,11 +34,25 @@
 namespace pvfmm_b200 {
 namespace {
 
-constexpr int kBM = 128, kBN = 64, kBK = 16;
+constexpr int kBN = 64, kBK = 16;
 constexpr int kAStride = kBK + 4;  // doubles per A row in shared memory
 constexpr int kBStride = kBN + 4;  // doubles per B row in shared memory (B fragment loads conflict-free)
 constexpr int kThreadsG = 256;
-constexpr int kSmemG = (int)sizeof(double) * (2 * kBM * kAStride + 2 * kBK * kBStride) + (int)sizeof(long) * kBM;
+
+// A block tile of BM x 64: 8 warps in WM x (8 / WM), each MI x NJ MMA tiles of
+// 8 x 8; STAGES K-steps in shared memory.
+template <int BM_, int WM_, int STAGES_>
+struct GemmTile {
+  static constexpr int BM = BM_, WM = WM_, WN = 8 / WM_, STAGES = STAGES_;
+  static constexpr int MI = BM / WM / 8, NJ = kBN / WN / 8;
+  static constexpr int smem =
+      (int)sizeof(double) * STAGES * (BM * kAStride + kBK * kBStride) + (int)sizeof(long) * BM;
+};
+#ifndef PVFMM_GEMM_STAGES
+#define PVFMM_GEMM_STAGES 2
+#endif
+using LargeTile = GemmTile<128, 4, PVFMM_GEMM_STAGES>;
+using SmallTile = GemmTile<32, 2, 4>;
 
 __device__ __forceinline__ void cp16(void* smem, const void* gmem, bool valid) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -51,89 +70,90 @@ struct RowMap {
   __device__ __forceinline__ long operator()(long i) const { return rows ? (long)rows[i] : i; }
 };
 
+template <class Tile>
 __global__ void __launch_bounds__(kThreadsG, 2)
     translate_gemm_kernel(int M, int N, int K, const double* __restrict__ A, long lda, const int* __restrict__ arows,
                           const double* __restrict__ B, long ldb, double* __restrict__ C, long ldc,
                           const int* __restrict__ crows, const MKey* __restrict__ keys, int deg, int accumulate,
                           long m_base, int kchunk, double* __restrict__ partial) {
+  constexpr int BM = Tile::BM, MI = Tile::MI, NJ = Tile::NJ, STAGES = Tile::STAGES;
   extern __shared__ __align__(16) double tsm[];
-  double(*As)[kBM * kAStride] = reinterpret_cast<double(*)[kBM * kAStride]>(tsm);
-  double(*Bs)[kBK * kBStride] = reinterpret_cast<double(*)[kBK * kBStride]>(tsm + 2 * kBM * kAStride);
-  long* arow_s = reinterpret_cast<long*>(tsm + 2 * kBM * kAStride + 2 * kBK * kBStride);
+  double(*As)[BM * kAStride] = reinterpret_cast<double(*)[BM * kAStride]>(tsm);
+  double(*Bs)[kBK * kBStride] = reinterpret_cast<double(*)[kBK * kBStride]>(tsm + STAGES * BM * kAStride);
+  long* arow_s = reinterpret_cast<long*>(tsm + STAGES * (BM * kAStride + kBK * kBStride));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int wm = warp >> 1, wn = warp & 1;  // warp tile (32 rows) x (32 cols)
-  const long m0 = m_base + (long)blockIdx.y * kBM;
+  const int wm = warp / Tile::WN, wn = warp % Tile::WN;  // warp tile (8 MI rows) x (8 NJ cols)
+  const long m0 = m_base + (long)blockIdx.y * BM;
   const int n0 = blockIdx.x * kBN;
   const RowMap amap{arows};
   // split K: this block sums k in [kbeg, kend) (the whole of K without a split)
   const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-  if (tid < kBM) arow_s[tid] = m0 + tid < M ? amap(m0 + tid) : -1;
+  if (tid < BM) arow_s[tid] = m0 + tid < M ? amap(m0 + tid) : -1;
   __syncthreads();
-  // copy plan: A tile 128 rows x 16 doubles = 1024 chunks of 16 B, 4 per
-  // thread; B tile 16 rows x 64 doubles = 512 chunks, 2 per thread
-  auto issue = [&](int k0, int buf) {
+  // copy plan: A tile BM rows x 16 doubles in 16-byte chunks, B tile 16 rows x
+  // 64 doubles = 512 chunks, 2 per thread.  One group per K-step (empty past
+  // the last one).
+  const int nk = (kend - kbeg + kBK - 1) / kBK;
+  auto issue = [&](int ks) {
+    const int k0 = kbeg + ks * kBK, buf = ks % STAGES;
+    if (ks < nk) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int c = tid + u * kThreadsG;
-      const int r = c >> 3, kc = (c & 7) * 2;  // row, first double of the chunk
-      const long ar = arow_s[r];
-      const bool v = ar >= 0 && k0 + kc < kend;
-      const double* src = v ? A + ar * lda + k0 + kc : A;
-      cp16(&As[buf][r * kAStride + kc], src, v);
-    }
+      for (int u = 0; u < BM * 8 / kThreadsG; ++u) {
+        const int c = tid + u * kThreadsG;
+        const int r = c >> 3, kc = (c & 7) * 2;  // row, first double of the chunk
+        const long ar = arow_s[r];
+        const bool v = ar >= 0 && k0 + kc < kend;
+        const double* src = v ? A + ar * lda + k0 + kc : A;
+        cp16(&As[buf][r * kAStride + kc], src, v);
+      }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int c = tid + u * kThreadsG;
-      const int r = c >> 5, nc = (c & 31) * 2;
-      const bool v = k0 + r < kend && n0 + nc < N;
-      const double* src = v ? B + (long)(k0 + r) * ldb + n0 + nc : B;
-      cp16(&Bs[buf][r * kBStride + nc], src, v);
+      for (int u = 0; u < 2; ++u) {
+        const int c = tid + u * kThreadsG;
+        const int r = c >> 5, nc = (c & 31) * 2;
+        const bool v = k0 + r < kend && n0 + nc < N;
+        const double* src = v ? B + (long)(k0 + r) * ldb + n0 + nc : B;
+        cp16(&Bs[buf][r * kBStride + nc], src, v);
+      }
     }
     cp_commit();
   };
-  double acc[4][4][2];
+  double acc[MI][NJ][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  const int nk = (kend - kbeg + kBK - 1) / kBK;
-  issue(kbeg, 0);
+    for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll
+  for (int ks = 0; ks < STAGES - 1; ++ks) issue(ks);
   for (int ks = 0; ks < nk; ++ks) {
-    const int buf = ks & 1;
-    if (ks + 1 < nk) {
-      issue(kbeg + (ks + 1) * kBK, buf ^ 1);
-      cp_wait<1>();
-    } else {
-      cp_wait<0>();
-    }
-    __syncthreads();
-    const double* as = As[buf] + (wm * 32) * kAStride;
-    const double* bs = Bs[buf] + wn * 32;
+    cp_wait<STAGES - 2>();  // this thread's copies of step ks have landed
+    __syncthreads();        // everyone's have; everyone is done with step ks - 1, whose buffer is refilled
+    const double* as = As[ks % STAGES] + (wm * 8 * MI) * kAStride;
+    const double* bs = Bs[ks % STAGES] + wn * 8 * NJ;
 #pragma unroll
     for (int kk = 0; kk < kBK; kk += 4) {
-      double a[4], b[4];
+      double a[MI], b[NJ];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = as[(i * 8 + g) * kAStride + kk + t];
+      for (int i = 0; i < MI; ++i) a[i] = as[(i * 8 + g) * kAStride + kk + t];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = bs[(kk + t) * kBStride + j * 8 + g];
+      for (int j = 0; j < NJ; ++j) b[j] = bs[(kk + t) * kBStride + j * 8 + g];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j], a[i], b[j]);
+        for (int j = 0; j < NJ; ++j) dmma(acc[i][j], a[i], b[j]);
+      if (kk == 0) issue(ks + STAGES - 1);  // behind the step's first MMAs
     }
-    __syncthreads();  // buffer buf is refilled by the next step's issue
   }
   // epilogue: rows g (+8i), columns 2t, 2t+1 of each 8x8 tile
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long mi = m0 + wm * 32 + i * 8 + g;
+  for (int i = 0; i < MI; ++i) {
+    const long mi = m0 + wm * 8 * MI + i * 8 + g;
     if (mi >= M) continue;
     if (partial) {  // split K: plain partial sums, reduced by translate_reduce
       double* prow = partial + ((long)blockIdx.z * M + mi) * N;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int n = n0 + wn * 32 + j * 8 + 2 * t;
+      for (int j = 0; j < NJ; ++j) {
+        const int n = n0 + wn * 8 * NJ + j * 8 + 2 * t;
         if (n < N) *reinterpret_cast<double2*>(prow + n) = make_double2(acc[i][j][0], acc[i][j][1]);
       }
       continue;
@@ -143,8 +163,8 @@ __global__ void __launch_bounds__(kThreadsG, 2)
     const long cr = crows ? (long)crows[mi] : mi;
     double* crow = C + cr * ldc;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + wn * 32 + j * 8 + 2 * t;
+    for (int j = 0; j < NJ; ++j) {
+      const int n = n0 + wn * 8 * NJ + j * 8 + 2 * t;
       if (n >= N) continue;  // N is even: n < N implies n + 1 < N
       double2 v = make_double2(acc[i][j][0] * s, acc[i][j][1] * s);
       double2* p = reinterpret_cast<double2*>(crow + n);
@@ -185,17 +205,32 @@ void translate_gemm(cudaStream_t s, long M, int N, int K, const double* A, long 
   if ((N & 1) || (K & 1) || (lda & 1) || (ldb & 1) || (ldc & 1))
     throw std::runtime_error("translate_gemm: row lengths must be even (16-byte rows)");
   if (M >= (1L << 31)) throw std::runtime_error("translate_gemm: too many rows");
-  PVFMM_CUDA_CHECK(cudaFuncSetAttribute(translate_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG));
-  // the column tiles of one row tile are consecutive blocks (they share the
-  // A rows in L2); row tiles in launches of at most 65535
-  const long tiles = (M + kBM - 1) / kBM;
-  for (long t0 = 0; t0 < tiles; t0 += 65535) {
-    dim3 grid((unsigned)((N + kBN - 1) / kBN), (unsigned)std::min(65535L, tiles - t0), (unsigned)ksplit);
-    translate_gemm_kernel<<<grid, kThreadsG, kSmemG, s>>>((int)M, N, K, A, lda, arows, B, ldb, C, ldc, crows, scale_keys,
-                                                      deg, accumulate ? 1 : 0, t0 * kBM, K / ksplit,
-                                                      ksplit > 1 ? partial : nullptr);
-    PVFMM_CUDA_CHECK(cudaGetLastError());
-  }
+  // Rows per block tile: 128, or 32 when the 128-row tiles would not fill the
+  // two blocks that an SM holds; a product of few rows lasts as long as one
+  // tile, most of whose rows are padding on the coarse levels.  With the 32-row
+  // tiles up to 296 blocks (against none, and up to 148): 2k Laplace points U2U
+  // 0.089 -> 0.052 ms and D2D 0.085 -> 0.040; 200k Stokes-gradient points U2U
+  // 0.38 -> 0.23 (0.25) and D2D 1.22 -> 0.60 (0.80).
+#ifndef PVFMM_GEMM_SMALL
+#define PVFMM_GEMM_SMALL 296
+#endif
+  const long cols = (N + kBN - 1) / kBN;
+  auto run = [&](auto kernel, int bm, int smem) {
+    PVFMM_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // the column tiles of one row tile are consecutive blocks (they share the
+    // A rows in L2); row tiles in launches of at most 65535
+    const long tiles = (M + bm - 1) / bm;
+    for (long t0 = 0; t0 < tiles; t0 += 65535) {
+      dim3 grid((unsigned)cols, (unsigned)std::min(65535L, tiles - t0), (unsigned)ksplit);
+      kernel<<<grid, kThreadsG, smem, s>>>((int)M, N, K, A, lda, arows, B, ldb, C, ldc, crows, scale_keys, deg,
+                                           accumulate ? 1 : 0, t0 * bm, K / ksplit, ksplit > 1 ? partial : nullptr);
+      PVFMM_CUDA_CHECK(cudaGetLastError());
+    }
+  };
+  if ((M + LargeTile::BM - 1) / LargeTile::BM * cols * ksplit <= PVFMM_GEMM_SMALL)
+    run(translate_gemm_kernel<SmallTile>, SmallTile::BM, SmallTile::smem);
+  else
+    run(translate_gemm_kernel<LargeTile>, LargeTile::BM, LargeTile::smem);
   if (ksplit > 1) {
     translate_reduce<<<(unsigned)((M * N + 255) / 256), 256, 0, s>>>(M, N, ksplit, partial, arows, crows, scale_keys,
                                                                      deg, accumulate ? 1 : 0, C, ldc);
