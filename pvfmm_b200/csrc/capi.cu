@@ -64,7 +64,8 @@ void destroy_context(Context& c) {
                   &T.int_idx, &T.src_perm, &T.trg_perm, &T.src_key, &T.trg_key, &T.src_leaf, &T.trg_leaf, &T.sx,
                   &T.sy, &T.sz, &T.tx, &T.ty, &T.tz, &T.sleaf, &T.tleaf, &T.vsrc, &T.vtrg, &T.node2vsrc, &T.vtab, &T.vmask, &T.vmorton, &T.vunion, &T.vucount, &T.vlocal,
                   &T.xtrg, &T.x_off, &T.x_list, &T.p_off, &T.p_list, &T.w_off, &T.w_list, &T.p_img, &T.x_img,
-                  &T.w_img, &c.dops.bc, &c.dops.d2d_f2};
+                  &T.w_img, &T.up_rows, &T.up_counts, &T.up_mask, &T.dn_rows, &T.dn_counts, &T.dn_mask,
+                  &c.dops.bc, &c.dops.d2d_f2};
   for (DevBuf* b : tb) b->release();
   if (c.events_ready)
     for (auto& e : c.ev) cudaEventDestroy(e);

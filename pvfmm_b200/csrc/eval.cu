@@ -2539,6 +2539,13 @@ void evaluate_impl(Context& ctx, const void* den_in, const void* dl_in, bool den
       // with few parents still fill the GPU; the 8 pieces are added in order.
       ctx.n_launch += 2;
       double* part = ctx.tmp_c.as<double>((size_t)8 * ni * din);
+      if (T.up_lists) {  // the children with sources only
+        const ChildRows up{T.up_rows.get<int>() + T.int_off[d], T.up_counts.get<int>() + 8 * d, T.int_off[T.depth],
+                           T.up_mask.get<unsigned char>() + T.int_off[d]};
+        translate_up(s, ni, din, ue + (size_t)T.level_off[d + 1] * din, ctx.dops.u2u.get<double>(), ue,
+                     T.int_idx.get<int>() + T.int_off[d], part, up);
+        continue;
+      }
       translate_gemm(s, ni, din, 8 * din, ue + (size_t)T.level_off[d + 1] * din, 8 * din, nullptr,
                      ctx.dops.u2u.get<double>(), din, ue, din, T.int_idx.get<int>() + T.int_off[d], nullptr, false, 8,
                      part);
@@ -2602,18 +2609,28 @@ void evaluate_impl(Context& ctx, const void* den_in, const void* dl_in, bool den
   for (int d = 0; d < T.depth; ++d) {
     const long ni = T.n_internal[d];
     if (ni == 0) continue;
+    // the children with targets only, where many leaves are empty
+    const ChildRows dn{T.dn_rows.get<int>() + T.int_off[d], T.dn_counts.get<int>() + 8 * d, T.int_off[T.depth],
+                       nullptr};
+    double* children = dc + (size_t)T.level_off[d + 1] * dout;
     if (ctx.d2d_factored) {  // (parents' dc DC2DE0) over the kept directions, then DC2DE1 M_pe2c
       double* tp = ctx.tmp_c.as<double>((size_t)ni * rd);
       ctx.n_launch += 2;
       translate_gemm(s, ni, rd, dout, dc, dout, T.int_idx.get<int>() + T.int_off[d], ctx.dops.dc2de0.get<double>(),
                      rd, tp, rd, nullptr, nullptr, false);
-      translate_gemm(s, ni, 8 * dout, rd, tp, rd, nullptr, ctx.dops.d2d_f2.get<double>(), 8 * dout,
-                     dc + (size_t)T.level_off[d + 1] * dout, 8 * dout, nullptr, nullptr, true);
+      if (T.dn_lists)
+        translate_down(s, ni, dout, rd, tp, rd, nullptr, ctx.dops.d2d_f2.get<double>(), children, dn);
+      else
+        translate_gemm(s, ni, 8 * dout, rd, tp, rd, nullptr, ctx.dops.d2d_f2.get<double>(), 8 * dout, children,
+                       8 * dout, nullptr, nullptr, true);
     } else {
       ++ctx.n_launch;
-      translate_gemm(s, ni, 8 * dout, dout, dc, dout, T.int_idx.get<int>() + T.int_off[d],
-                     ctx.dops.d2d.get<double>(), 8 * dout, dc + (size_t)T.level_off[d + 1] * dout, 8 * dout, nullptr,
-                     nullptr, true);
+      if (T.dn_lists)
+        translate_down(s, ni, dout, dout, dc, dout, T.int_idx.get<int>() + T.int_off[d], ctx.dops.d2d.get<double>(),
+                       children, dn);
+      else
+        translate_gemm(s, ni, 8 * dout, dout, dc, dout, T.int_idx.get<int>() + T.int_off[d],
+                       ctx.dops.d2d.get<double>(), 8 * dout, children, 8 * dout, nullptr, nullptr, true);
     }
   }
   ev(8);

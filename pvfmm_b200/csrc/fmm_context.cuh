@@ -25,6 +25,10 @@ struct DevTree {
   DevBuf colleague;                   // int[27] per node
   DevBuf int_idx;                     // internal node ids, level by level (offsets int_off)
   std::vector<long> int_off;
+  // internal nodes whose children have sources / targets, per level and octant
+  // (ChildRows; built when many leaves are empty)
+  DevBuf up_rows, up_counts, up_mask, dn_rows, dn_counts, dn_mask;
+  bool up_lists = false, dn_lists = false;
   // point data (sorted)
   long n_src = 0, n_trg = 0;
   // point sets the source positions stand for: 1 per density passed
@@ -162,5 +166,27 @@ void hadamard_tc5_operator_layout(const std::vector<double>& vop, int n3h, std::
 void translate_gemm(cudaStream_t s, long M, int N, int K, const double* A, long lda, const int* arows,
                     const double* B, long ldb, double* C, long ldc, const int* crows, const MKey* scale_keys,
                     bool accumulate, int ksplit = 1, double* partial = nullptr, int deg = 1);
+
+// Products between the parents of a level and their children that leave out
+// the children without points: per octant z the indices k of the parents whose
+// child z has some, rows[z stride ..] with counts[z] of them (on the device),
+// and per parent the mask of those octants.
+struct ChildRows {
+  const int* rows;
+  const int* counts;
+  long stride;
+  const unsigned char* mask;
+};
+// C[crows[k]] = sum over the octants z in the mask of children[8k + z] B_z, in
+// octant order (U2U; `partial`: 8 M din doubles)
+void translate_up(cudaStream_t s, long M, int din, const double* children, const double* B, double* C,
+                  const int* crows, double* partial, const ChildRows& lists);
+// children[8k + z] += A[arows(k)] B_z for the listed (k, z) (D2D)
+void translate_down(cudaStream_t s, long M, int dout, int K, const double* A, long lda, const int* arows,
+                    const double* B, double* children, const ChildRows& lists);
+// Whether translate_down is the cheaper form when `occupied` of `all` leaves
+// have points: it starts a column tile at every octant (dout = 152: 192
+// columns for 152), which the plain product over all 8 octants does not.
+bool translate_down_pays(long occupied, long all, int dout);
 
 }  // namespace pvfmm_b200

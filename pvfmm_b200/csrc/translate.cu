@@ -70,12 +70,19 @@ struct RowMap {
   __device__ __forceinline__ long operator()(long i) const { return rows ? (long)rows[i] : i; }
 };
 
-template <class Tile>
+// Over parents and children (kUp, kDown; see ChildRows): blockIdx.z is the
+// child octant, the rows are the listed parents' indices k.
+// kUp: A's rows are the parents' blocks of 8 child rows, of which octant z is
+// the K range [z kchunk, (z + 1) kchunk); kDown: B's and C's columns
+// [z N, (z + 1) N).
+enum GemmMode { kPlainRows, kUp, kDown };
+
+template <class Tile, GemmMode Mode>
 __global__ void __launch_bounds__(kThreadsG, 2)
     translate_gemm_kernel(int M, int N, int K, const double* __restrict__ A, long lda, const int* __restrict__ arows,
                           const double* __restrict__ B, long ldb, double* __restrict__ C, long ldc,
                           const int* __restrict__ crows, const MKey* __restrict__ keys, int deg, int accumulate,
-                          long m_base, int kchunk, double* __restrict__ partial) {
+                          long m_base, int kchunk, double* __restrict__ partial, ChildRows lists) {
   constexpr int BM = Tile::BM, MI = Tile::MI, NJ = Tile::NJ, STAGES = Tile::STAGES;
   extern __shared__ __align__(16) double tsm[];
   double(*As)[BM * kAStride] = reinterpret_cast<double(*)[BM * kAStride]>(tsm);
@@ -87,9 +94,16 @@ __global__ void __launch_bounds__(kThreadsG, 2)
   const long m0 = m_base + (long)blockIdx.y * BM;
   const int n0 = blockIdx.x * kBN;
   const RowMap amap{arows};
+  const int* listed = Mode == kPlainRows ? nullptr : lists.rows + blockIdx.z * lists.stride;
+  const int rows = Mode == kPlainRows ? M : lists.counts[blockIdx.z];
+  if (Mode != kPlainRows && m0 >= rows) return;
+  if (Mode == kDown) {
+    B += (long)blockIdx.z * N;
+    C += (long)blockIdx.z * N;
+  }
   // split K: this block sums k in [kbeg, kend) (the whole of K without a split)
-  const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-  if (tid < BM) arow_s[tid] = m0 + tid < M ? amap(m0 + tid) : -1;
+  const int kbeg = Mode == kDown ? 0 : blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
+  if (tid < BM) arow_s[tid] = m0 + tid < rows ? amap(listed ? listed[m0 + tid] : m0 + tid) : -1;
   __syncthreads();
   // copy plan: A tile BM rows x 16 doubles in 16-byte chunks, B tile 16 rows x
   // 64 doubles = 512 chunks, 2 per thread.  One group per K-step (empty past
@@ -148,9 +162,10 @@ __global__ void __launch_bounds__(kThreadsG, 2)
 #pragma unroll
   for (int i = 0; i < MI; ++i) {
     const long mi = m0 + wm * 8 * MI + i * 8 + g;
-    if (mi >= M) continue;
+    if (mi >= rows) continue;
+    const long out_row = listed ? listed[mi] : mi;
     if (partial) {  // split K: plain partial sums, reduced by translate_reduce
-      double* prow = partial + ((long)blockIdx.z * M + mi) * N;
+      double* prow = partial + ((long)blockIdx.z * M + out_row) * N;
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
         const int n = n0 + wn * 8 * NJ + j * 8 + 2 * t;
@@ -160,7 +175,7 @@ __global__ void __launch_bounds__(kThreadsG, 2)
     }
     double s = 1.0;
     if (keys) s = ldexp(1.0, -deg * (int)(keys[arow_s[mi - m0]].lo & 31u));
-    const long cr = crows ? (long)crows[mi] : mi;
+    const long cr = crows ? (long)crows[out_row] : out_row;
     double* crow = C + cr * ldc;
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
@@ -182,13 +197,15 @@ __global__ void __launch_bounds__(kThreadsG, 2)
 __global__ void translate_reduce(long M, int N, int ksplit, const double* __restrict__ partial,
                                  const int* __restrict__ arows, const int* __restrict__ crows,
                                  const MKey* __restrict__ keys, int deg, int accumulate, double* __restrict__ C,
-                                 long ldc) {
+                                 long ldc, const unsigned char* __restrict__ mask) {
   const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (e >= M * N) return;
   const long i = e / N;
   const int n = (int)(e % N);
   double v = 0;
-  for (int z = 0; z < ksplit; ++z) v += partial[((long)z * M + i) * N + n];
+  const unsigned m = mask ? mask[i] : ~0u;  // (the pieces of a child without a row were not formed)
+  for (int z = 0; z < ksplit; ++z)
+    if (m >> z & 1u) v += partial[((long)z * M + i) * N + n];
   if (keys) v *= ldexp(1.0, -deg * (int)(keys[arows ? arows[i] : i].lo & 31u));
   double* c = C + (crows ? (long)crows[i] : i) * ldc + n;
   *c = accumulate ? *c + v : v;
@@ -196,24 +213,22 @@ __global__ void translate_reduce(long M, int N, int ksplit, const double* __rest
 
 }  // namespace
 
-void translate_gemm(cudaStream_t s, long M, int N, int K, const double* A, long lda, const int* arows,
-                    const double* B, long ldb, double* C, long ldc, const int* crows, const MKey* scale_keys,
-                    bool accumulate, int ksplit, double* partial, int deg) {
-  if (M <= 0 || N <= 0) return;
-  if (ksplit < 1 || (ksplit > 1 && (!partial || K % ksplit != 0 || (K / ksplit) % 2 != 0)))
-    throw std::runtime_error("translate_gemm: bad K split");
-  if ((N & 1) || (K & 1) || (lda & 1) || (ldb & 1) || (ldc & 1))
-    throw std::runtime_error("translate_gemm: row lengths must be even (16-byte rows)");
-  if (M >= (1L << 31)) throw std::runtime_error("translate_gemm: too many rows");
-  // Rows per block tile: 128, or 32 when the 128-row tiles would not fill the
-  // two blocks that an SM holds; a product of few rows lasts as long as one
-  // tile, most of whose rows are padding on the coarse levels.  With the 32-row
-  // tiles up to 296 blocks (against none, and up to 148): 2k Laplace points U2U
-  // 0.089 -> 0.052 ms and D2D 0.085 -> 0.040; 200k Stokes-gradient points U2U
-  // 0.38 -> 0.23 (0.25) and D2D 1.22 -> 0.60 (0.80).
+// Rows per block tile: 128, or 32 when the 128-row tiles would not fill the
+// two blocks that an SM holds; a product of few rows lasts as long as one tile,
+// most of whose rows are padding on the coarse levels.  With the 32-row tiles
+// up to 296 blocks (against none, and up to 148): 2k Laplace points U2U 0.089
+// -> 0.052 ms and D2D 0.085 -> 0.040; 200k Stokes-gradient points U2U 0.38 ->
+// 0.23 (0.25) and D2D 1.22 -> 0.60 (0.80).
 #ifndef PVFMM_GEMM_SMALL
 #define PVFMM_GEMM_SMALL 296
 #endif
+template <GemmMode Mode>
+static void launch_gemm(cudaStream_t s, long M, int N, int K, const double* A, long lda, const int* arows,
+                        const double* B, long ldb, double* C, long ldc, const int* crows, const MKey* scale_keys,
+                        bool accumulate, int nz, int kchunk, double* partial, int deg, const ChildRows& lists) {
+  if ((N & 1) || (K & 1) || (kchunk & 1) || (lda & 1) || (ldb & 1) || (ldc & 1))
+    throw std::runtime_error("translate_gemm: row lengths must be even (16-byte rows)");
+  if (M >= (1L << 31)) throw std::runtime_error("translate_gemm: too many rows");
   const long cols = (N + kBN - 1) / kBN;
   auto run = [&](auto kernel, int bm, int smem) {
     PVFMM_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -221,21 +236,53 @@ void translate_gemm(cudaStream_t s, long M, int N, int K, const double* A, long 
     // A rows in L2); row tiles in launches of at most 65535
     const long tiles = (M + bm - 1) / bm;
     for (long t0 = 0; t0 < tiles; t0 += 65535) {
-      dim3 grid((unsigned)cols, (unsigned)std::min(65535L, tiles - t0), (unsigned)ksplit);
+      dim3 grid((unsigned)cols, (unsigned)std::min(65535L, tiles - t0), (unsigned)nz);
       kernel<<<grid, kThreadsG, smem, s>>>((int)M, N, K, A, lda, arows, B, ldb, C, ldc, crows, scale_keys, deg,
-                                           accumulate ? 1 : 0, t0 * bm, K / ksplit, ksplit > 1 ? partial : nullptr);
+                                           accumulate ? 1 : 0, t0 * bm, kchunk, partial, lists);
       PVFMM_CUDA_CHECK(cudaGetLastError());
     }
   };
-  if ((M + LargeTile::BM - 1) / LargeTile::BM * cols * ksplit <= PVFMM_GEMM_SMALL)
-    run(translate_gemm_kernel<SmallTile>, SmallTile::BM, SmallTile::smem);
+  if ((M + LargeTile::BM - 1) / LargeTile::BM * cols * nz <= PVFMM_GEMM_SMALL)
+    run(translate_gemm_kernel<SmallTile, Mode>, SmallTile::BM, SmallTile::smem);
   else
-    run(translate_gemm_kernel<LargeTile>, LargeTile::BM, LargeTile::smem);
+    run(translate_gemm_kernel<LargeTile, Mode>, LargeTile::BM, LargeTile::smem);
+}
+
+void translate_gemm(cudaStream_t s, long M, int N, int K, const double* A, long lda, const int* arows,
+                    const double* B, long ldb, double* C, long ldc, const int* crows, const MKey* scale_keys,
+                    bool accumulate, int ksplit, double* partial, int deg) {
+  if (M <= 0 || N <= 0) return;
+  if (ksplit < 1 || (ksplit > 1 && (!partial || K % ksplit != 0 || (K / ksplit) % 2 != 0)))
+    throw std::runtime_error("translate_gemm: bad K split");
+  launch_gemm<kPlainRows>(s, M, N, K, A, lda, arows, B, ldb, C, ldc, crows, scale_keys, accumulate, ksplit, K / ksplit,
+                          ksplit > 1 ? partial : nullptr, deg, ChildRows{});
   if (ksplit > 1) {
     translate_reduce<<<(unsigned)((M * N + 255) / 256), 256, 0, s>>>(M, N, ksplit, partial, arows, crows, scale_keys,
-                                                                     deg, accumulate ? 1 : 0, C, ldc);
+                                                                     deg, accumulate ? 1 : 0, C, ldc, nullptr);
     PVFMM_CUDA_CHECK(cudaGetLastError());
   }
+}
+
+void translate_up(cudaStream_t s, long M, int din, const double* children, const double* B, double* C,
+                  const int* crows, double* partial, const ChildRows& lists) {
+  if (M <= 0) return;
+  launch_gemm<kUp>(s, M, din, 8 * din, children, 8L * din, nullptr, B, din, C, din, nullptr, nullptr, false, 8, din,
+                   partial, 1, lists);
+  translate_reduce<<<(unsigned)((M * din + 255) / 256), 256, 0, s>>>(M, din, 8, partial, nullptr, crows, nullptr, 1, 0,
+                                                                     C, din, lists.mask);
+  PVFMM_CUDA_CHECK(cudaGetLastError());
+}
+
+void translate_down(cudaStream_t s, long M, int dout, int K, const double* A, long lda, const int* arows,
+                    const double* B, double* children, const ChildRows& lists) {
+  if (M <= 0) return;
+  launch_gemm<kDown>(s, M, dout, K, A, lda, arows, B, 8L * dout, children, 8L * dout, nullptr, nullptr, true, 8, K,
+                     nullptr, 1, lists);
+}
+
+bool translate_down_pays(long occupied, long all, int dout) {
+  const double padded = (double)((dout + kBN - 1) / kBN * kBN) / dout;
+  return occupied * padded < 0.85 * all;
 }
 
 }  // namespace pvfmm_b200
@@ -280,6 +327,52 @@ extern "C" int PVFMMB200TranslateGemmCheck(long M, int N, int K, const double* A
     return 0;
   } catch (const std::exception& e) {
     if (buf) cudaFree(buf);
+    set_last_error(e.what());
+    return 1;
+  }
+}
+
+// Self-check of the parent-child products (internal entry point used by the
+// GPU tests; no counterpart in the reference): with the children of parent k
+// in the bits of mask[k], up[k] = sum over those children z of children[8k + z]
+// B_z (B: 8 dim x dim) and down[8k + z] += up_in[k] D_z (D: dim x 8 dim), on
+// device copies of the host arrays.  Returns 0 on success.
+extern "C" int PVFMMB200ChildProductsCheck(long M, int dim, const unsigned char* mask, const double* children,
+                                           const double* B, double* up, const double* up_in, const double* D,
+                                           double* down) {
+  using namespace pvfmm_b200;
+  DevBuf b[8];
+  try {
+    std::vector<int> rows(8 * M, -1), counts(8, 0);
+    for (long k = 0; k < M; ++k)
+      for (int z = 0; z < 8; ++z)
+        if (mask[k] >> z & 1) rows[z * M + counts[z]++] = (int)k;
+    auto put = [&](DevBuf& d, const void* h, size_t bytes) {
+      d.ensure(bytes);
+      PVFMM_CUDA_CHECK(cudaMemcpy(d.ptr, h, bytes, cudaMemcpyHostToDevice));
+    };
+    const size_t n1 = (size_t)M * dim * 8, n8 = 8 * n1, nb = (size_t)64 * dim * dim;
+    put(b[0], rows.data(), rows.size() * sizeof(int));
+    put(b[1], counts.data(), 8 * sizeof(int));
+    put(b[2], mask, M);
+    put(b[3], children, n8);
+    put(b[4], B, nb);
+    put(b[5], up, n1);
+    const ChildRows lists{b[0].get<int>(), b[1].get<int>(), M, b[2].get<unsigned char>()};
+    translate_up(nullptr, M, dim, b[3].get<double>(), b[4].get<double>(), b[5].get<double>(), nullptr,
+                 b[6].as<double>(n8 / 8), lists);
+    PVFMM_CUDA_CHECK(cudaMemcpy(up, b[5].ptr, n1, cudaMemcpyDeviceToHost));
+    put(b[5], up_in, n1);
+    put(b[4], D, nb);
+    put(b[7], down, n8);
+    translate_down(nullptr, M, dim, dim, b[5].get<double>(), dim, nullptr, b[4].get<double>(), b[7].get<double>(),
+                   lists);
+    PVFMM_CUDA_CHECK(cudaMemcpy(down, b[7].ptr, n8, cudaMemcpyDeviceToHost));
+    for (DevBuf& d : b) d.release();
+    set_last_error("");
+    return 0;
+  } catch (const std::exception& e) {
+    for (DevBuf& d : b) d.release();
     set_last_error(e.what());
     return 1;
   }

@@ -413,6 +413,36 @@ __global__ void gather_coords(const double* __restrict__ in, const int* __restri
   out[i * 3 + 2] = in[p * 3 + 2];
 }
 
+// Rows of the parent-child products (ChildRows): internal node j (index k in
+// its level) joins, for every octant z whose child has points [lo, hi), the
+// list of its level and octant.  The order within a list is the order of
+// arrival; every row's product is formed by itself, so it changes no value.
+__global__ void child_rows(LevelTab lt, long n_int, const int* __restrict__ int_idx, const int* __restrict__ child0,
+                           const int* __restrict__ lo, const int* __restrict__ hi, int* __restrict__ rows,
+                           int* __restrict__ counts, unsigned char* __restrict__ mask) {
+  const long j = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  int d = 0;
+  const bool in = j < n_int;
+  while (in && d + 1 < lt.depth && j >= lt.ioff[d + 1]) ++d;
+  const int lane = threadIdx.x & 31;
+  const unsigned same = __match_any_sync(0xffffffffu, in ? d : -1);
+  const int c0 = in ? child0[int_idx[j]] : 0;
+  unsigned m = 0;
+  for (int z = 0; z < 8; ++z) {
+    const bool has = in && hi[c0 + z] > lo[c0 + z];
+    const unsigned vote = __ballot_sync(0xffffffffu, has) & same;  // the lanes of this level with a row
+    int base = 0;
+    const int leader = __ffs(vote) - 1;
+    if (has && lane == leader) base = atomicAdd(&counts[d * 8 + z], __popc(vote));
+    base = __shfl_sync(0xffffffffu, base, vote ? leader : 0);
+    if (has) {
+      m |= 1u << z;
+      rows[z * n_int + lt.ioff[d] + base + __popc(vote & ((1u << lane) - 1))] = (int)(j - lt.ioff[d]);
+    }
+  }
+  if (in) mask[j] = (unsigned char)m;
+}
+
 // ------------------------------------------------------------------ lists
 // Image of colleague c at slot ci of node v (periodic boundaries): the
 // shift, in units of the unit cube, that moves c to the slot's position next
@@ -1154,6 +1184,28 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
       localize<double><<<ceil_div(T.n_tleaf, 4), 128, 0, s>>>(T.tleaf.get<int>(), T.n_tleaf, keys, tlo, thi,
                                                              coords_t.get<double>(), tx, ty, tz, tl);
     }
+  }
+  // 11. rows of the parent-child products where enough leaves are empty and
+  //     the tree is large enough for the products to outlast their launches
+  //     (2M surface points, 38k internal nodes, 62% of the leaves empty: U2U
+  //     2.19 -> 1.14 ms, D2D 2.08 -> 1.10; 150k surface points with 2k internal
+  //     nodes: U2U 0.127 -> 0.122, D2D 0.101 -> 0.117, and 0.02 for the lists)
+  T.up_lists = T.dn_lists = false;
+  if (n_int_total >= 4096) {
+    const long leaves = N - n_int_total;
+    auto lists = [&](const int* lo, const int* hi, DevBuf& rows, DevBuf& counts, DevBuf& mask) {
+      int* r = rows.as<int>(8 * n_int_total);
+      int* c = counts.as<int>(8 * kMaxDepth);
+      unsigned char* m = mask.as<unsigned char>(n_int_total);
+      PVFMM_CUDA_CHECK(cudaMemsetAsync(c, 0, 8 * kMaxDepth * sizeof(int), s));
+      ++ctx.n_launch;
+      child_rows<<<ceil_div(n_int_total, 128), 128, 0, s>>>(lt, n_int_total, int_idx, child0, lo, hi, r, c, m);
+    };
+    // U2U's products have no padding to pay for: a list at 15% empty leaves
+    T.up_lists = T.src_counted && T.n_sleaf < 0.85 * leaves;
+    if (T.up_lists) lists(slo, shi, T.up_rows, T.up_counts, T.up_mask);
+    T.dn_lists = translate_down_pays(T.n_tleaf, leaves, ctx.ns * ctx.hops.kout);
+    if (T.dn_lists) lists(tlo, thi, T.dn_rows, T.dn_counts, T.dn_mask);
   }
   PVFMM_CUDA_CHECK(cudaGetLastError());
   T.valid = true;  // the evaluation is queued behind the last kernels
