@@ -945,6 +945,31 @@ __device__ __forceinline__ Cplx<Real> csub(const Cplx<Real>& a, const Cplx<Real>
 template <class Real>
 __device__ __forceinline__ Cplx<Real> cmuli(const Cplx<Real>& a) { return {-a.im, a.re}; }
 
+// Output z = M + zp of the length-2M inverse DFT as a plain sum (twr, twi:
+// cos and sin of 2 pi j / 2M in shared memory).  FP32 keeps this form: the
+// rounding of these sums is the largest part of the mixed form's V-list error,
+// and position gradients near leaf corners carry it amplified (up to 4e-5 at
+// m = 10), so that the radix-4 sums, although their error was a fifth smaller
+// (and the inverse 1.37 -> 0.78 ms at 4M clustered points), moved such outputs
+// by more than two forms of the other stages differ.
+// Literal: the twiddles as literal operands instead, which blocks of whole rows
+// take (4M clustered points 1.37 against 1.83 ms; smaller blocks are faster
+// from shared memory, 1M Stokes 0.52 against 0.62 ms).
+template <class Real, int M, bool Literal>
+__device__ __forceinline__ Cplx<Real> idft_plain(const Cplx<Real> (&v)[2 * M], int zp, const Real* twr,
+                                                 const Real* twi) {
+  constexpr Twiddles<Real, 2 * M> tw{};
+  Real re = 0, im = 0;
+#pragma unroll
+  for (int k = 0; k < 2 * M; ++k) {
+    const int w = (k * (M + zp)) % (2 * M);
+    const Real c = Literal ? tw.c[w] : twr[w], s = Literal ? tw.s[w] : twi[w];
+    re += v[k].re * c - v[k].im * s;
+    im += v[k].re * s + v[k].im * c;
+  }
+  return {re, im};
+}
+
 // Four outputs of the length-2M DFT of M values, X[k0 + j M/2], j = 0..3
 // (k0 < M/2): the values' classes y mod 4 are summed once, S_r = sum of
 // v[y] w^(k0 y) over y = r (mod 4), w = exp(-pi i / M), and since w^(y M/2) =
@@ -1000,10 +1025,11 @@ struct FftSizes {
 
 // Each stage of the separable DFTs: one thread per input line; it loads the
 // line into registers once and writes every output along that axis (radix-4
-// sums along y and z, paired outputs kx and M - kx along x, literal twiddles).
+// sums along y and z, paired outputs kx and M - kx along x, literal twiddles;
+// plain sums in the FP32 inverse, see idft_plain).
 // Against plain sums with the twiddles in shared memory, piece-major FP64
 // spectra and 4-byte FP16 stores, 4M clustered points in the mixed form:
-// forward 1.73 -> 0.99 ms, inverse 1.62 -> 0.78 ms; 1M in FP64: 1.89 -> 0.64
+// forward 1.73 -> 0.99 ms, inverse 1.62 -> 1.37 ms; 1M in FP64: 1.89 -> 0.64
 // and 0.95 -> 0.56 ms.  What bounds the forward one now is its 64-byte row
 // stores at the frequency-major stride.
 // Output layout: frequency-major rows (split_row) for the scalar FP64
@@ -1046,8 +1072,6 @@ __global__ void __launch_bounds__(576) fft_up_kernel(int ke, int G, int ngroups,
     Real v[M];
 #pragma unroll
     for (int x = 0; x < M; ++x) v[x] = row[x];
-    // sums over even and odd x give both X[kx] = E + O and, since
-    // w^((M - kx) x) = (-1)^x conj(w^(kx x)), X[M - kx] = conj(E - O)
     constexpr Twiddles<Real, N1> tw{};
 #pragma unroll
     for (int kx = 0; kx <= M / 2; ++kx) {
@@ -1128,7 +1152,7 @@ __global__ void __launch_bounds__(576) fft_up_kernel(int ke, int G, int ngroups,
   }
 }
 
-template <class Real, int M>
+template <class Real, int M, bool Literal>
 __global__ void __launch_bounds__(576) ifft_dn_kernel(int ke, int G, int ngroups, const int* __restrict__ vtrg,
                                                        const int* __restrict__ child0, const MKey* __restrict__ keys,
                                                        const Cplx<Real>* __restrict__ spec,
@@ -1141,6 +1165,8 @@ __global__ void __launch_bounds__(576) ifft_dn_kernel(int ke, int G, int ngroups
   Cplx<Real>* b1 = reinterpret_cast<Cplx<Real>*>(smem_raw);  // G * B1S
   Cplx<Real>* b2 = b1 + G * B1S;                             // G * M*M*NH
   Real* o = reinterpret_cast<Real*>(b1);                     // G * M3, once b1 has been read
+  Real* twr = reinterpret_cast<Real*>(b2 + G * M * M * NH);  // FP32: twiddles
+  Real* twi = twr + N1;
   const int vt = blockIdx.x / ngroups;
   const int gb = (blockIdx.x % ngroups) * G;
   const int ngrid = 8 * ke;
@@ -1151,6 +1177,15 @@ __global__ void __launch_bounds__(576) ifft_dn_kernel(int ke, int G, int ngroups
   decode_key(keys[P], X, Y, Z, dP);
   const double lscale = ldexp(1.0, deg * ((int)dP + 1));  // 2^(trg_scal * level of the children)
   const int dim = ns * ke;
+  if constexpr (sizeof(Real) == 4 && !Literal) {
+    for (int j = threadIdx.x; j < N1; j += blockDim.x) {
+      double sn, cs;
+      sincospi(2.0 * j / N1, &sn, &cs);
+      twr[j] = (Real)cs;
+      twi[j] = (Real)sn;
+    }
+    __syncthreads();
+  }
   const Cplx<Real>* in = spec + (long)vt * (N1 * NH * nkz) * ngrid + gb;
   // kz -> z in [M, 2M): line = (gi, ky, kx) read straight from the spectrum
   // row of the parent (gi fastest: neighbouring threads read neighbouring
@@ -1158,6 +1193,15 @@ __global__ void __launch_bounds__(576) ifft_dn_kernel(int ke, int G, int ngroups
   // slab's frequencies alone is added into dc (the transform is linear).
   for (int i = threadIdx.x; i < gn * N1 * NH; i += blockDim.x) {
     const int gi = i % gn, l = i / gn;  // l = ky*NH + kx
+    if constexpr (sizeof(Real) == 4) {
+      Cplx<Real> v[N1];
+#pragma unroll
+      for (int kz = 0; kz < N1; ++kz)
+        v[kz] = (kz >= kz0 && kz < kz0 + nkz) ? in[(long)(l + N1 * NH * (kz - kz0)) * ngrid + gi] : Cplx<Real>{0, 0};
+#pragma unroll
+      for (int zp = 0; zp < M; ++zp) b1[gi * B1S + zp * N1 * NH + l] = idft_plain<Real, M, Literal>(v, zp, twr, twi);
+      continue;
+    }
     Cplx<Real> acc[M] = {};
 #pragma unroll
     for (int k0 = 0; k0 < M / 2; ++k0) {
@@ -1177,6 +1221,14 @@ __global__ void __launch_bounds__(576) ifft_dn_kernel(int ke, int G, int ngroups
   for (int i = threadIdx.x; i < gn * M * NH; i += blockDim.x) {
     const int kx = i % NH, zg = i / NH;  // zg = gi*M + zp
     const Cplx<Real>* col = b1 + (zg / M) * B1S + ((zg % M) * N1) * NH + kx;
+    if constexpr (sizeof(Real) == 4) {
+      Cplx<Real> v[N1];
+#pragma unroll
+      for (int ky = 0; ky < N1; ++ky) v[ky] = col[ky * NH];
+#pragma unroll
+      for (int yp = 0; yp < M; ++yp) b2[(zg * M + yp) * NH + kx] = idft_plain<Real, M, Literal>(v, yp, twr, twi);
+      continue;
+    }
     Cplx<Real> acc[M] = {};
 #pragma unroll
     for (int k0 = 0; k0 < M / 2; ++k0) {
@@ -1192,9 +1244,27 @@ __global__ void __launch_bounds__(576) ifft_dn_kernel(int ke, int G, int ngroups
   // kx -> x in [M, 2M), c2r: line = (gi, zp, yp)
   for (int r = threadIdx.x; r < gn * M * M; r += blockDim.x) {
     const Cplx<Real>* row = b2 + r * NH;
+    constexpr Twiddles<Real, N1> tw{};
+    if constexpr (sizeof(Real) == 4) {
+      Cplx<Real> v[NH];
+#pragma unroll
+      for (int kx = 0; kx < NH; ++kx) v[kx] = row[kx];
+#pragma unroll
+      for (int xp = 0; xp < M; ++xp) {
+        Real acc = 0;
+#pragma unroll
+        for (int kx = 0; kx < NH; ++kx) {
+          const int w = (kx * (M + xp)) % N1;
+          const Real c = Literal ? tw.c[w] : twr[w], sn = Literal ? tw.s[w] : twi[w];
+          const Real t = v[kx].re * c - v[kx].im * sn;
+          acc += (kx == 0 || 2 * kx == N1) ? t : (Real)2 * t;
+        }
+        o[r * M + xp] = acc;
+      }
+      continue;
+    }
     // y[xp] = sum over kx of (2 for 0 < kx < M) (-1)^kx Re(v[kx] W^(kx xp));
     // kx and M - kx share cos and sin up to the sign (-1)^xp
-    constexpr Twiddles<Real, N1> tw{};
     Cplx<Real> even[M / 2], odd[M / 2];
 #pragma unroll
     for (int kx = 0; kx < M / 2; ++kx) {
@@ -2259,17 +2329,17 @@ void vlist_fft_t(Context& ctx, const double* ue, double* dc, Cplx<Real>* sin_, C
   // two blocks of 112 KB share an SM: the FP32 scalar DFTs of m = 8 take all 8
   // children and so write (read) whole 64-byte rows of the spectra; forward,
   // 4M clustered points, 0.99 ms against 1.30 ms with 4 children in 60 KB.
-  // The inverse gains only for those (0.85 -> 0.78 ms; the others are slower
-  // in large blocks: 1M Stokes m = 6 0.34 ms in 288 threads, 0.40 in 448).
+  // The inverse gains only for those (1.62 -> 1.37 ms); the others are slower
+  // in large blocks.
   const int Gu = grids_per_block<F>(F::up_grid_bytes, ngrid_up, 112 * 1024, 576);
   const size_t sm_up = Gu * F::up_grid_bytes;
   PVFMM_CUDA_CHECK(cudaFuncSetAttribute(fft_up_kernel<Real, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_up));
   const bool rows = sizeof(Real) == 4 && ngrid_dn == 8 && 8 * F::dn_grid_bytes <= 112 * 1024;
   const int Gd = rows ? grids_per_block<F>(F::dn_grid_bytes, ngrid_dn, 112 * 1024, 576)
                       : grids_per_block<F>(F::dn_grid_bytes, ngrid_dn, 80 * 1024, 288);
-  const size_t sm_dn = Gd * F::dn_grid_bytes;
-  PVFMM_CUDA_CHECK(
-      cudaFuncSetAttribute(ifft_dn_kernel<Real, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_dn));
+  const size_t sm_dn = Gd * F::dn_grid_bytes + 2 * F::N1 * sizeof(Real);
+  const auto ifft = rows ? ifft_dn_kernel<Real, M, true> : ifft_dn_kernel<Real, M, false>;
+  PVFMM_CUDA_CHECK(cudaFuncSetAttribute(ifft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_dn));
   // split-FP16 input spectra for the mixed form's tensor-core Hadamards
   const double* qinv = nullptr;
   if (sizeof(Real) == 4 && !(kin == 1 ? use_tc5(ctx) : use_simt3())) {
@@ -2316,7 +2386,7 @@ void vlist_fft_t(Context& ctx, const double* ue, double* dc, Cplx<Real>* sin_, C
       }
       if (p0 == 0 && sl == 0) ev(5);
       ++ctx.n_launch;
-      ifft_dn_kernel<Real, M><<<np * (ngrid_dn / Gd), F::threads(Gd), sm_dn, s>>>(
+      ifft<<<np * (ngrid_dn / Gd), F::threads(Gd), sm_dn, s>>>(
           kout, Gd, ngrid_dn / Gd, T.vtrg.get<int>() + p0, T.child0.get<int>(), T.key.get<MKey>(), sout,
           ctx.dops.ifft_map.get<int>(), ctx.ns, ctx.ki.deg, kz0, nkz, dc);
     }
