@@ -6,7 +6,7 @@ full FMM -- of the Laplace potential+gradient kernel on N = 4,000,000 points
 drawn from a mixture of 8 isotropic Gaussians (sigma 0.02, centres uniform in
 [0.1,0.9]^3, clipped to [0,1]^3), sources = targets, densities uniform
 [-1,1], multipole order 8, at most 256 points per leaf.  Both forms run:
-plain FP64 and mixed (FP32 near field and V-list DFTs, split-TF32 tensor-core
+plain FP64 and mixed (FP32 near field and V-list DFTs, split-FP16 tensor-core
 V-list products, FP64 check->equivalent chain).  Each form's error is the
 relative L2 error of all 4 outputs against an FP64 direct sum over all
 sources on 2,000 sampled targets; ``value`` is the targets/s of the fastest
@@ -454,9 +454,9 @@ TRAFFIC_1M = {
     ("near_field", 8): {"bytes": 151890688 + 20192256, "units": 1000000},        # near_field_kernel<double>
 }
 # kernel that computes the V-list Hadamard products: (real bytes, ke) -> name
-HADAMARD_KERNEL = {(4, 1): "hadamard_tc_kernel (V-list M2L, TF32 mma.sync x3 split)",
+HADAMARD_KERNEL = {(4, 1): "hadamard_tc_kernel (V-list M2L, FP16 mma.sync x3 split)",
                    (8, 1): "hadamard_dmma1_kernel (V-list M2L, FP64 mma.sync m8n8k4)",
-                   (4, 3): "hadamard_tc3_kernel<3> (V-list M2L, TF32 mma.sync x3 split)",
+                   (4, 3): "hadamard_tc3_kernel<3> (V-list M2L, FP16 mma.sync x3 split)",
                    (8, 3): "hadamard_dmma3_kernel<3> (V-list M2L, FP64 mma.sync m8n8k4)"}
 NEAR_KERNEL = "near_field_kernel (U-list P2P + W + D2T)"
 
@@ -475,8 +475,8 @@ def roofline(B, peaks):
       (n_vsrc + n_vtrg) * n3h * 8 children * 2 * rb (input spectra read once,
       output spectra written once) + 26 * n3h * 64 * 2 * rb (operators read
       once) against the measured copy bandwidth; its tensor view (mixed form:
-      the split issues 3 TF32 products per product, against a dense TF32 peak
-      of half the measured bf16 peak) or FP64 tensor view (plain form, against
+      the split issues 3 FP16 products per product, against the measured dense
+      bf16 peak, the FP16 rate) or FP64 tensor view (plain form, against
       the nominal FP64 peak, the same for the FP64 tensor cores and the FP64
       pipe) is the `compute` sub-object.
     `traffic` is the ncu DRAM traffic of a launch scaled from 1M points."""
@@ -484,7 +484,7 @@ def roofline(B, peaks):
     rb = B["real_bytes"]
     hbm_peak = peaks.get("hbm_gbs", 6650.0)
     peak_src = "measured" if "hbm_gbs" in peaks else "fallback"
-    tf32_peak = peaks.get("bf16_tflops", 1590.0) / 2
+    fp16_peak = peaks.get("bf16_tflops", 1590.0)
     smax = (B["clocks"] or {}).get("sm_max_mhz") or 1965.0
     lanes = 128 if rb == 4 else 64
     simt_peak = 148 * lanes * 2 * smax * 1e6 / 1e12
@@ -508,8 +508,9 @@ def roofline(B, peaks):
            "frac": had_gbs / hbm_peak, "peak_source": peak_src,
            "traffic": traffic("hadamard", st["n_vsrc"] + st["n_vtrg"]), "algorithmic_bytes": had_bytes,
            "kernel_ms": had_ms,
-           "compute": ({"pipe": "tensor tf32 x3 (mma.sync)", "achieved_tflops": 3 * had_tf, "peak_tflops": tf32_peak,
-                        "peak_source": "half the measured bf16 dense peak", "frac": 3 * had_tf / tf32_peak,
+           "compute": ({"pipe": "tensor fp16 x3 (mma.sync)", "achieved_tflops": 3 * had_tf, "peak_tflops": fp16_peak,
+                        "peak_source": "the measured bf16 dense peak" if "bf16_tflops" in peaks else "fallback",
+                        "frac": 3 * had_tf / fp16_peak,
                         "algorithmic_flops": had_flops} if tensor else
                        {"pipe": "fp64 tensor (mma.sync m8n8k4)", "achieved_tflops": had_tf,
                         "peak_tflops": simt_peak, "peak_source": "nominal", "frac": had_tf / simt_peak,

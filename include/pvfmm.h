@@ -118,7 +118,7 @@ enum PVFMMPrecision {
                                 Newton step, hi+lo coordinates, partial sums
                                 promoted to FP64 every 16 sources), FP32
                                 V-list DFTs, V-list products on the tensor
-                                cores as 3-term split TF32; FP64 for the
+                                cores as 3-term split FP16; FP64 for the
                                 check-to-equivalent chain (S2U and X check
                                 potentials, pseudo-inverse GEMMs, U2U, D2D,
                                 D2T evaluation) */
