@@ -844,9 +844,12 @@ __device__ __forceinline__ long split_row(int f, long q, long n_q) { return (lon
 __device__ __forceinline__ int split_word(int e) { return (e >> 1) * 4 + (e & 1); }
 
 // Exponents of the parents' spectra: |spectrum value| <= sum |density| of its
-// child, so E = (exponent of the largest such sum over the 8 children) - 15;
-// qscale = 2^E, qinv = 2^-E.  One block of 8 warps per parent, one child per
-// warp; `len` values per child.  A sum that is zero or not finite leaves E = 0.
+// child, so E = (exponent of the largest such sum over the 8 children) - 15,
+// but at least -126: below that 2^-E would leave the range of FP64 (densities
+// near 1e-304 and less), and lo's step 2^(E-24) is finer there than FP32's
+// smallest step 2^-149.  qscale = 2^E, qinv = 2^-E.  One block of 8 warps per
+// parent, one child per warp; `len` values per child.  A sum that is zero or
+// not finite leaves E = 0.
 __global__ void __launch_bounds__(256) vsrc_scale_kernel(const int* __restrict__ vsrc, const int* __restrict__ child0,
                                                          const double* __restrict__ ue, int len,
                                                          float* __restrict__ qscale, double* __restrict__ qinv) {
@@ -868,8 +871,9 @@ __global__ void __launch_bounds__(256) vsrc_scale_kernel(const int* __restrict__
     }
     int e = 15;
     if (finite && top > 0) frexp(top, &e);
-    qscale[blockIdx.x] = (float)ldexp(1.0, e - 15);
-    qinv[blockIdx.x] = ldexp(1.0, 15 - e);
+    e = max(e - 15, -126);
+    qscale[blockIdx.x] = (float)ldexp(1.0, e);
+    qinv[blockIdx.x] = ldexp(1.0, -e);
   }
 }
 

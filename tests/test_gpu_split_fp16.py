@@ -25,6 +25,15 @@ def _rel(a, b):
     return np.linalg.norm(a - b) / np.linalg.norm(b)
 
 
+def _compare(monkeypatch, kernel, m, x, q):
+    """The mixed form's outputs and what they are held against."""
+    a = _ctx(kernel, m).evaluate(x, q, None, x, True)
+    if P.KERNEL_DIMS[kernel][0] == 1:
+        return a, _ctx(kernel, m, P.PRECISION_PLAIN).evaluate(x, q, None, x, True)
+    monkeypatch.setenv("PVFMM_B200_HADAMARD3", "simt")
+    return a, _ctx(kernel, m).evaluate(x, q, None, x, True)
+
+
 @pytest.mark.parametrize("kernel,m", KERNELS)
 @pytest.mark.parametrize("k", [-70, 70])
 def test_power_of_two_densities_scale_the_output_exactly(kernel, m, k):
@@ -35,6 +44,26 @@ def test_power_of_two_densities_scale_the_output_exactly(kernel, m, k):
     a = ctx.evaluate(x, q, None, x, True)
     b = ctx.evaluate(x, np.ldexp(q, k), None, x, False)
     assert np.array_equal(b, np.ldexp(a, k))
+
+
+# Densities that FP32 rounds to zero (Gaussian weights far out: 1e-306, and
+# subnormal FP64 numbers) beside ordinary ones, and alone: 2^-E of such a
+# parent has no finite value.
+@pytest.mark.parametrize("kernel,m", KERNELS)
+@pytest.mark.parametrize("alone", [False, True])
+def test_densities_below_the_fp32_range(monkeypatch, kernel, m, alone):
+    rng = np.random.default_rng(8)
+    pos = rng.random((3001, 3))
+    q = rng.standard_normal((3001, P.KERNEL_DIMS[kernel][0]))
+    q[pos[:, 0] < 0.5] *= 1e-306
+    q[pos[:, 0] < 0.25] *= 1e-14
+    x = pos.reshape(-1)
+    if alone:
+        q[pos[:, 0] >= 0.5] = 0.0
+        assert np.all(np.abs(_ctx(kernel, m).evaluate(x, q.reshape(-1), None, x, True)) < 1e-290)
+        return
+    a, b = _compare(monkeypatch, kernel, m, x, q.reshape(-1))
+    assert _rel(a, b) < 1e-6
 
 
 # 600 / 1500 / 5001 points: 1 V-list target parent below a full tile of 16,
