@@ -847,11 +847,13 @@ __device__ __forceinline__ int split_word(int e) { return (e >> 1) * 4 + (e & 1)
 // child, so E = (exponent of the largest such sum over the 8 children) - 15,
 // but at least -126: below that 2^-E would leave the range of FP64 (densities
 // near 1e-304 and less), and lo's step 2^(E-24) is finer there than FP32's
-// smallest step 2^-149.  qscale = 2^E, qinv = 2^-E.  One block of 8 warps per
+// smallest step 2^-149.  qinv = 2^-E; qscale = 2^(E + op_exp) also carries the
+// operators' largest scale, so that the running sums of the products are at
+// most as large as the largest output spectra allow.  One block of 8 warps per
 // parent, one child per warp; `len` values per child.  A sum that is zero or
 // not finite leaves E = 0.
 __global__ void __launch_bounds__(256) vsrc_scale_kernel(const int* __restrict__ vsrc, const int* __restrict__ child0,
-                                                         const double* __restrict__ ue, int len,
+                                                         const double* __restrict__ ue, int len, int op_exp,
                                                          float* __restrict__ qscale, double* __restrict__ qinv) {
   __shared__ double part[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -872,7 +874,7 @@ __global__ void __launch_bounds__(256) vsrc_scale_kernel(const int* __restrict__
     int e = 15;
     if (finite && top > 0) frexp(top, &e);
     e = max(e - 15, -126);
-    qscale[blockIdx.x] = (float)ldexp(1.0, e);
+    qscale[blockIdx.x] = (float)ldexp(1.0, e + op_exp);
     qinv[blockIdx.x] = ldexp(1.0, -e);
   }
 }
@@ -2350,7 +2352,8 @@ void vlist_fft_t(Context& ctx, const double* ue, double* dc, Cplx<Real>* sin_, C
     float* qs = ctx.qscale.as<float>(T.n_vsrc);
     double* qi = ctx.qinv.as<double>(T.n_vsrc);
     ++ctx.n_launch;
-    vsrc_scale_kernel<<<T.n_vsrc, 256, 0, s>>>(T.vsrc.get<int>(), T.child0.get<int>(), ue, ctx.ns * kin, qs, qi);
+    vsrc_scale_kernel<<<T.n_vsrc, 256, 0, s>>>(T.vsrc.get<int>(), T.child0.get<int>(), ue, ctx.ns * kin,
+                                             ctx.vop_exp, qs, qi);
     qinv = qi;
   }
   // slabs of kz (the slowest frequency index): each slab's forward DFT rows,
@@ -2765,6 +2768,7 @@ void evaluate_impl(Context& ctx, const void* den_in, const void* dl_in, bool den
 
 // Exponents of the operators per frequency: fscale[f] = 2^(E - 14) with every
 // |re|, |im| of frequency f below 2^E, so that the fragments stay below 2^14.
+// (upload_vop_fragments then moves the largest of them to the parents' scales.)
 __global__ void __launch_bounds__(256) vop_scale_kernel(int n, const float2* __restrict__ vop,
                                                         float* __restrict__ fscale) {
   __shared__ float part[256];
@@ -2892,6 +2896,18 @@ static void upload_vop_fragments(Context& ctx) {
   vop_scale_kernel<<<n3h, 256, 0, ctx.stream>>>(26 * 64 * ki * ko, ctx.dops.vop.get<float2>(), fs);
   vop_fragments_kernel<<<ceil_div(n, 256L), 256, 0, ctx.stream>>>(n, ki, ko, koc, ctx.dops.vop.get<float2>(), fs, dev);
   PVFMM_CUDA_CHECK(cudaGetLastError());
+  // The largest scale 2^vop_exp goes to the source parents (vsrc_scale_kernel):
+  // the Hadamards' sums before fscale[f] <= 1 then stay within the bound of the
+  // largest output spectra.  Summed in units of the scaled operators they left
+  // the FP32 range at densities 2^18 to 2^20 smaller (about 1e31).  -23 keeps the
+  // smallest parent scale, 2^(-126 + vop_exp), representable.
+  std::vector<float> hfs(n3h);
+  PVFMM_CUDA_CHECK(cudaMemcpyAsync(hfs.data(), fs, n3h * sizeof(float), cudaMemcpyDeviceToHost, ctx.stream));
+  PVFMM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
+  std::frexp(*std::max_element(hfs.begin(), hfs.end()), &ctx.vop_exp);
+  ctx.vop_exp = std::max(ctx.vop_exp - 1, -23);
+  for (float& v : hfs) v = std::ldexp(v, -ctx.vop_exp);
+  PVFMM_CUDA_CHECK(cudaMemcpyAsync(fs, hfs.data(), n3h * sizeof(float), cudaMemcpyHostToDevice, ctx.stream));
   PVFMM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
 }
 

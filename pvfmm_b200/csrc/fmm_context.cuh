@@ -71,7 +71,7 @@ struct DevTree {
 struct DevOps {
   DevBuf uc2ue0, uc2ue1, dc2de0, dc2de1, u2u, d2d, vop;
   DevBuf vop_frag;  // Hadamard operators as MMA fragments (mixed form: split FP16, plain form: FP64)
-  DevBuf vop_fscale;  // mixed form: power-of-two scale of the fragments per frequency
+  DevBuf vop_fscale;  // mixed form: power-of-two scale of the fragments per frequency, over 2^Context::vop_exp
   DevBuf vop_tc5;   // mixed form, ke = 1: Hadamard operators in the tcgen05 shared-memory layout
   DevBuf ue_basis;  // mixed Stokes form: din x r32, the upward directions above the FP32 cutoff
   DevBuf bc;        // periodic boundaries: din x dout, root upward equivalent -> root downward check
@@ -118,6 +118,7 @@ struct Context {
   DevBuf uc_c, tmp_c, de_c;  // compact GEMM buffers
   DevBuf spec_in, spec_out;  // V-list spectra
   DevBuf qscale, qinv;       // mixed form: power-of-two scale of each V-list source parent's spectra
+  int vop_exp = 0;           // mixed form: exponent of the operators' largest scale (part of qscale)
   DevBuf scratch;         // sort / scan temporaries
   DevBuf scratch2;
   DevBuf io_src, io_trg, io_den, io_val;  // staging for host-pointer calls

@@ -46,6 +46,21 @@ def test_power_of_two_densities_scale_the_output_exactly(kernel, m, k):
     assert np.array_equal(b, np.ldexp(a, k))
 
 
+# Densities up to where the near field's q/r itself leaves the FP32 range, and
+# down to where the smallest output spectra do: the scales of the stored halves
+# must not overflow or vanish before that.
+@pytest.mark.parametrize("kernel,m", [(P.FMMKernel.LaplacePotential, 8), (P.FMMKernel.StokesVelocity, 4)])
+@pytest.mark.parametrize("k", [-90, 112])
+def test_whole_fp32_range_of_densities(kernel, m, k):
+    rng = np.random.default_rng(6)
+    x = rng.random(3 * 3001)
+    q = rng.uniform(0.5, 1.0, 3001 * P.KERNEL_DIMS[kernel][0])
+    ctx = _ctx(kernel, m)
+    a = ctx.evaluate(x, q, None, x, True)
+    b = ctx.evaluate(x, np.ldexp(q, k), None, x, False)
+    assert np.array_equal(b, np.ldexp(a, k))
+
+
 # Densities that FP32 rounds to zero (Gaussian weights far out: 1e-306, and
 # subnormal FP64 numbers) beside ordinary ones, and alone: 2^-E of such a
 # parent has no finite value.
