@@ -1027,6 +1027,30 @@ struct FftSizes {
   static constexpr int B1S = M * N1 * NH + 4;
   static constexpr size_t dn_grid_bytes = sizeof(Real) * 2 * (B1S + M * M * NH);
   static constexpr int threads(int G) { return ((8 * NH * G + 31) / 32) * 32; }  // one thread per line of the widest stage
+  // Grids per block: the largest divisor G of ngrid with G grids in `budget`
+  // bytes and at most max_threads threads (at least 1).
+  static constexpr int grids_per_block(size_t per_grid, int ngrid, size_t budget, int max_threads) {
+    int best = 1;
+    for (int G = 1; G <= ngrid; ++G)
+      if (ngrid % G == 0 && G * per_grid <= budget && threads(G) <= max_threads) best = G;
+    return best;
+  }
+  // Two blocks of 112 KB share an SM: the FP32 scalar DFTs of m = 8 take all 8
+  // children and so write (read) whole 64-byte rows of the spectra; forward,
+  // 4M clustered points, 0.99 ms against 1.30 ms with 4 children in 60 KB.
+  // The inverse gains only for those (kRows; 1.62 -> 1.37 ms); the others are
+  // slower in large blocks.
+  static constexpr int up_grids(int ngrid) { return grids_per_block(up_grid_bytes, ngrid, 112 * 1024, 576); }
+  static constexpr bool kRows = sizeof(Real) == 4 && 8 * dn_grid_bytes <= 112 * 1024;  // FP32 up to m = 8
+  static constexpr int dn_grids(int ngrid) {
+    return kRows && ngrid == 8 ? grids_per_block(dn_grid_bytes, ngrid, 112 * 1024, 576)
+                               : grids_per_block(dn_grid_bytes, ngrid, 80 * 1024, 288);
+  }
+  // Launch bound of the forward kernel, for 8 and 24 grids: 576 threads hold it
+  // to 96 registers, too few for the lines of m >= 14 in FP64, whose blocks
+  // need far fewer threads (200k points, m = 14 1.10 against 1.02 ms, m = 16
+  // 1.57 against 1.47).
+  static constexpr int up_bound = threads(up_grids(8)) <= 288 && threads(up_grids(24)) <= 288 ? 288 : 576;
 };
 
 // Each stage of the separable DFTs: one thread per input line; it loads the
@@ -1043,7 +1067,7 @@ struct FftSizes {
 // each value times 2^-E of its parent as FP16 hi + lo in the order of
 // split_word; otherwise rows spec[q][f][child*ke+comp].
 template <class Real, int M>
-__global__ void __launch_bounds__(576) fft_up_kernel(int ke, int G, int ngroups, const int* __restrict__ vsrc,
+__global__ void __launch_bounds__(FftSizes<Real, M>::up_bound) fft_up_kernel(int ke, int G, int ngroups, const int* __restrict__ vsrc,
                                                       const int* __restrict__ child0, const double* __restrict__ ue,
                                                       const int* __restrict__ fft_map, int ns, long n_q, int kz0,
                                                       int nkz, const double* __restrict__ qinv,
@@ -1158,12 +1182,17 @@ __global__ void __launch_bounds__(576) fft_up_kernel(int ke, int G, int ngroups,
   }
 }
 
+// Literal blocks hold whole rows (kRows) in up to 576 threads, the others up to
+// 288.  Above m = 10 the bound is what the blocks have, so that the lines keep
+// their registers (FP32: 126 at m = 12 to 153 at m = 16): held to 96 they
+// spilled up to 1.1 KB, mixed inverse at 200k points, m = 12 0.427 ms against
+// 0.362, m = 16 2.05 against 1.37.  At m = 10 the 96 registers lack 4 bytes and
+// are the faster form (0.163 ms against 0.177 with 102).
 template <class Real, int M, bool Literal>
-__global__ void __launch_bounds__(576) ifft_dn_kernel(int ke, int G, int ngroups, const int* __restrict__ vtrg,
-                                                       const int* __restrict__ child0, const MKey* __restrict__ keys,
-                                                       const Cplx<Real>* __restrict__ spec,
-                                                       const int* __restrict__ ifft_map, int ns, int deg, int kz0,
-                                                       int nkz, double* __restrict__ dc) {
+__global__ void __launch_bounds__(Literal || M <= 10 ? 576 : 288)
+    ifft_dn_kernel(int ke, int G, int ngroups, const int* __restrict__ vtrg, const int* __restrict__ child0,
+                   const MKey* __restrict__ keys, const Cplx<Real>* __restrict__ spec,
+                   const int* __restrict__ ifft_map, int ns, int deg, int kz0, int nkz, double* __restrict__ dc) {
   using F = FftSizes<Real, M>;
   constexpr int N1 = F::N1, NH = F::NH, M3 = F::M3, N3H = F::N3H;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2286,17 +2315,6 @@ void upload_vec(DevBuf& b, const std::vector<double>& v, cudaStream_t s) {
   PVFMM_CUDA_CHECK(cudaStreamSynchronize(s));
 }
 
-// Grids per block of the DFT kernels: the largest divisor G of ngrid with
-// G*per_grid <= budget and at most max_threads for threads(G) (at least 1;
-// the kernels are bounded to 576 threads).
-template <class F>
-int grids_per_block(size_t per_grid, int ngrid, size_t budget, int max_threads) {
-  int best = 1;
-  for (int G = 1; G <= ngrid; ++G)
-    if (ngrid % G == 0 && G * per_grid <= budget && F::threads(G) <= max_threads) best = G;
-  return best;
-}
-
 // V-list: forward DFTs of every source parent, then the Hadamard products
 // and inverse DFTs of the target parents in chunks of `chunk` parents (the
 // output spectra of one chunk at a time; one chunk when device memory
@@ -2332,19 +2350,14 @@ void vlist_fft_t(Context& ctx, const double* ue, double* dc, Cplx<Real>* sin_, C
   auto s = ctx.stream;
   using F = FftSizes<Real, M>;
   const int ngrid_up = 8 * kin, ngrid_dn = 8 * kout;
-  // two blocks of 112 KB share an SM: the FP32 scalar DFTs of m = 8 take all 8
-  // children and so write (read) whole 64-byte rows of the spectra; forward,
-  // 4M clustered points, 0.99 ms against 1.30 ms with 4 children in 60 KB.
-  // The inverse gains only for those (1.62 -> 1.37 ms); the others are slower
-  // in large blocks.
-  const int Gu = grids_per_block<F>(F::up_grid_bytes, ngrid_up, 112 * 1024, 576);
+  const int Gu = F::up_grids(ngrid_up), Gd = F::dn_grids(ngrid_dn);
   const size_t sm_up = Gu * F::up_grid_bytes;
   PVFMM_CUDA_CHECK(cudaFuncSetAttribute(fft_up_kernel<Real, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_up));
-  const bool rows = sizeof(Real) == 4 && ngrid_dn == 8 && 8 * F::dn_grid_bytes <= 112 * 1024;
-  const int Gd = rows ? grids_per_block<F>(F::dn_grid_bytes, ngrid_dn, 112 * 1024, 576)
-                      : grids_per_block<F>(F::dn_grid_bytes, ngrid_dn, 80 * 1024, 288);
   const size_t sm_dn = Gd * F::dn_grid_bytes + 2 * F::N1 * sizeof(Real);
-  const auto ifft = rows ? ifft_dn_kernel<Real, M, true> : ifft_dn_kernel<Real, M, false>;
+  auto ifft = ifft_dn_kernel<Real, M, false>;
+  if constexpr (F::kRows) {
+    if (ngrid_dn == 8) ifft = ifft_dn_kernel<Real, M, true>;
+  }
   PVFMM_CUDA_CHECK(cudaFuncSetAttribute(ifft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_dn));
   // split-FP16 input spectra for the mixed form's tensor-core Hadamards
   const double* qinv = nullptr;
@@ -3048,3 +3061,50 @@ void evaluate(Context& ctx, const void* den_in, const void* dl_in, bool den_floa
 }
 
 }  // namespace pvfmm_b200
+
+namespace {
+template <class Real, int M>
+void dft_local_bytes(int* up, int* dn) {
+  using namespace pvfmm_b200;
+  cudaFuncAttributes a{};
+  PVFMM_CUDA_CHECK(cudaFuncGetAttributes(&a, fft_up_kernel<Real, M>));
+  *up = (int)a.localSizeBytes;
+  PVFMM_CUDA_CHECK(cudaFuncGetAttributes(&a, ifft_dn_kernel<Real, M, false>));
+  *dn = (int)a.localSizeBytes;
+  if constexpr (FftSizes<Real, M>::kRows) {
+    PVFMM_CUDA_CHECK(cudaFuncGetAttributes(&a, ifft_dn_kernel<Real, M, true>));
+    *dn = std::max(*dn, (int)a.localSizeBytes);
+  }
+}
+}  // namespace
+
+// Local memory per thread of the V-list DFT kernels of a form (0 plain, 1
+// mixed) and order, forward and inverse: what of a line did not fit the
+// registers (internal entry point used by the GPU tests; no counterpart in the
+// reference).  Returns 0 on success.
+extern "C" int PVFMMB200DftLocalBytes(int precision, int m, int* up, int* dn) {
+  using pvfmm_b200::set_last_error;
+  try {
+    auto get = [&](auto order) {
+      constexpr int M = decltype(order)::value;
+      if (precision == 0) dft_local_bytes<double, M>(up, dn);
+      else dft_local_bytes<float, M>(up, dn);
+    };
+    switch (m) {
+      case 2: get(std::integral_constant<int, 2>()); break;
+      case 4: get(std::integral_constant<int, 4>()); break;
+      case 6: get(std::integral_constant<int, 6>()); break;
+      case 8: get(std::integral_constant<int, 8>()); break;
+      case 10: get(std::integral_constant<int, 10>()); break;
+      case 12: get(std::integral_constant<int, 12>()); break;
+      case 14: get(std::integral_constant<int, 14>()); break;
+      case 16: get(std::integral_constant<int, 16>()); break;
+      default: throw std::runtime_error("unsupported multipole order");
+    }
+    set_last_error("");
+    return 0;
+  } catch (const std::exception& e) {
+    set_last_error(e.what());
+    return 1;
+  }
+}
