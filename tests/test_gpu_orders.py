@@ -40,3 +40,21 @@ def test_dft_lines_stay_in_registers(prec, m):
     up, dn = ctypes.c_int(-1), ctypes.c_int(-1)
     assert f(int(prec), m, ctypes.byref(up), ctypes.byref(dn)) == 0, P.last_error()
     assert (up.value, dn.value) == (0, 0)
+
+
+def test_mixed_potentials_at_order_10():
+    """The V-list's FP32 rounding shows most at m = 10.  Median relative error
+    of the potentials against the plain form, geometric mean over eight point
+    sets: 2.05e-7 with chained FP32 sums along x, 2.38e-7 with paired ones
+    (higher in each set).  The bar lies between."""
+    logs = []
+    ctx = [P.FMMParticleContext(-1, 120, 10, P.FMMKernel.LaplacePotential, precision=p)
+           for p in (P.PRECISION_MIXED, P.PRECISION_PLAIN)]
+    for seed in range(8):
+        rng = np.random.default_rng(seed)
+        centres = rng.uniform(0.1, 0.9, (8, 3))
+        x = np.clip(centres[rng.integers(0, 8, 100_000)] + 0.02 * rng.standard_normal((100_000, 3)), 0, 1).reshape(-1)
+        q = rng.uniform(-1, 1, 100_000)
+        a, b = (c.evaluate(x, q, None, x, True) for c in ctx)
+        logs.append(np.log(np.median(np.abs(a - b) / np.abs(b))))
+    assert np.exp(np.mean(logs)) < 2.2e-7
