@@ -1579,9 +1579,9 @@ __global__ void __launch_bounds__(128, 4) hadamard_rd_kernel(int n3h, long n_vtr
 
 // ---------------------------------------------------------------------------
 // Hadamard products of the mixed form (scalar expansions here, 3-component
-// ones below) on the tensor cores: mma.sync m16n8k16 on split-FP16 spectra and operators with FP32 accumulation, three products
-// per value (a_lo b_hi + a_hi b_lo + a_hi b_hi), which carries the products to
-// ~2^-22 relative.
+// ones below) on the tensor cores: mma.sync m16n8k16 on split-FP16 spectra and
+// operators with FP32 accumulation, three products per value (a_lo b_hi +
+// a_hi b_lo + a_hi b_hi), which carries the products to ~2^-22 relative.
 //
 // Per frequency f the product is a real GEMM over parent rows:
 //   OUT[P][(e_out, re|im)] += sum_o sum_(e, re|im) IN[Q_o(P)][(e, re|im)] * B_o[(e, re|im)][(e_out, re|im)]
@@ -1637,28 +1637,19 @@ __device__ __forceinline__ void mma_split(float (&d)[4], const uint4& x, const u
   mma_f16(d, x.x, y.x, x.y, y.y, b.x, b.y);
 }
 
-#ifndef PVFMM_TC_WARPS
-#define PVFMM_TC_WARPS 8
-#endif
-constexpr int kTcWarps = PVFMM_TC_WARPS;  // warps per block of the scalar tensor-core Hadamard
-#ifndef PVFMM_TC_MIN_BLOCKS
-#define PVFMM_TC_MIN_BLOCKS 3
-#endif
-#ifndef PVFMM_TC_CHUNKS
-#define PVFMM_TC_CHUNKS 16  // tiles per warp (operator fragments staged once)
-#endif
+constexpr int kTcWarps = 8;    // warps per block of the scalar tensor-core Hadamard
+constexpr int kTcBlocks = 3;   // blocks per SM
+constexpr int kTcStages = 3;   // register sets of gathered rows
+constexpr int kTcChunks = 16;  // tiles per warp (operator fragments staged once)
 
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
 }
 
-#ifndef PVFMM_TC_STAGES
-#define PVFMM_TC_STAGES 3
-#endif
 constexpr int kTcEnt = 26 * 16 + 16;  // words of a tile's table: source parents [26][16], patterns [16]
 
-__global__ void __launch_bounds__(32 * kTcWarps, PVFMM_TC_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * kTcWarps, kTcBlocks)
     hadamard_tc_kernel(int n3h, long n_vtrg, long vt_stride, long n_vsrc, int chunks, const int* __restrict__ vtab,
                        const unsigned* __restrict__ vmask, const uint4* __restrict__ spec_in,
                        const float* __restrict__ qscale, const uint4* __restrict__ bfrag,
@@ -1731,7 +1722,7 @@ __global__ void __launch_bounds__(32 * kTcWarps, PVFMM_TC_MIN_BLOCKS)
     // The tile's occupied offsets in increasing order, one set bit at a time,
     // kStages register sets in turn: the gathers of the next offsets are in
     // flight while one is multiplied.
-    constexpr int kStages = PVFMM_TC_STAGES;
+    constexpr int kStages = kTcStages;
     const int nlive = __popc(rem);
     Rows r[kStages];
     int o[kStages];
@@ -1776,22 +1767,17 @@ __global__ void __launch_bounds__(32 * kTcWarps, PVFMM_TC_MIN_BLOCKS)
 // target parents; lane (g, t) loads the 16-byte pieces 4u + t, u = 0..2, of
 // the 192-byte rows g and g+8.  The B fragments of an offset (9 KB for KOC =
 // 3) are too many to stage for all 26 offsets, so the block streams them,
-// PVFMM_TC3_OPB offsets at a time, into a double buffer in shared memory
+// kTc3Opb offsets at a time, into a double buffer in shared memory
 // (cp.async, one barrier per group), shared by its 8 warps; offsets that no
 // parent of the block has are skipped, those that no parent of a warp has are
 // skipped by that warp.  Each k-step accumulates in a fresh fragment.
 // ---------------------------------------------------------------------------
 constexpr int kTc3Warps = 8;
-#ifndef PVFMM_TC3_OPB
-#define PVFMM_TC3_OPB 4  // offsets whose B fragments are staged per barrier (1M Stokes points: 2 6.22, 4 6.14 ms)
-#endif
-constexpr int kTc3Opb = PVFMM_TC3_OPB;
-#ifndef PVFMM_TC3_MIN_BLOCKS
-#define PVFMM_TC3_MIN_BLOCKS 2
-#endif
+constexpr int kTc3Blocks = 2;  // blocks per SM
+constexpr int kTc3Opb = 4;  // offsets whose B fragments are staged per barrier (1M Stokes points: 2 6.22, 4 6.14 ms)
 
 template <int KOC>
-__global__ void __launch_bounds__(32 * kTc3Warps, PVFMM_TC3_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * kTc3Warps, kTc3Blocks)
     hadamard_tc3_kernel(int n3h, long n_vtrg, long vt_stride, long n_vsrc, int ko, const int* __restrict__ vtab,
                         const unsigned* __restrict__ vmask, const uint4* __restrict__ spec_in,
                         const float* __restrict__ qscale, const uint4* __restrict__ bfrag,
@@ -2203,7 +2189,7 @@ void launch_hadamard_tc(Context& ctx, int n3h, long f_base, const Cplx<float>* s
   DevTree& T = ctx.tree;
   const size_t sm = (size_t)26 * 2 * 32 * sizeof(uint4) + (size_t)kTcWarps * 2 * kTcEnt * sizeof(int);
   PVFMM_CUDA_CHECK(cudaFuncSetAttribute(hadamard_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  const int chunks = PVFMM_TC_CHUNKS;
+  const int chunks = kTcChunks;
   dim3 grid(ceil_div(np, (long)16 * kTcWarps * chunks), n3h);
   ++ctx.n_launch;
   hadamard_tc_kernel<<<grid, 32 * kTcWarps, sm, ctx.stream>>>(
@@ -2401,7 +2387,7 @@ void vlist_fft_t(Context& ctx, const double* ue, double* dc, Cplx<Real>* sin_, C
         }
         else if (use_tc5(ctx)) launch_hadamard_tc5(ctx, n3h, f_base, sin_, sout, p0, np);
         else launch_hadamard_tc(ctx, n3h, f_base, sin_, sout, p0, np);
-      } else if (!use_simt3()) {  // 3-component expansions: tensor cores (TF32 x3 or FP64)
+      } else if (!use_simt3()) {  // 3-component expansions: tensor cores (split FP16 or FP64)
         if constexpr (sizeof(Real) == 4) {
           if (kout == 1) launch_hadamard_tc3<1>(ctx, n3h, f_base, 1, sin_, sout, p0, np);
           else launch_hadamard_tc3<3>(ctx, n3h, f_base, kout, sin_, sout, p0, np);

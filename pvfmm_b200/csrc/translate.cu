@@ -48,10 +48,7 @@ struct GemmTile {
   static constexpr int smem =
       (int)sizeof(double) * STAGES * (BM * kAStride + kBK * kBStride) + (int)sizeof(long) * BM;
 };
-#ifndef PVFMM_GEMM_STAGES
-#define PVFMM_GEMM_STAGES 2
-#endif
-using LargeTile = GemmTile<128, 4, PVFMM_GEMM_STAGES>;
+using LargeTile = GemmTile<128, 4, 2>;
 using SmallTile = GemmTile<32, 2, 4>;
 
 __device__ __forceinline__ void cp16(void* smem, const void* gmem, bool valid) {
@@ -219,9 +216,7 @@ __global__ void translate_reduce(long M, int N, int ksplit, const double* __rest
 // up to 296 blocks (against none, and up to 148): 2k Laplace points U2U 0.089
 // -> 0.052 ms and D2D 0.085 -> 0.040; 200k Stokes-gradient points U2U 0.38 ->
 // 0.23 (0.25) and D2D 1.22 -> 0.60 (0.80).
-#ifndef PVFMM_GEMM_SMALL
-#define PVFMM_GEMM_SMALL 296
-#endif
+constexpr long kSmallTileBlocks = 296;
 template <GemmMode Mode>
 static void launch_gemm(cudaStream_t s, long M, int N, int K, const double* A, long lda, const int* arows,
                         const double* B, long ldb, double* C, long ldc, const int* crows, const MKey* scale_keys,
@@ -242,7 +237,7 @@ static void launch_gemm(cudaStream_t s, long M, int N, int K, const double* A, l
       PVFMM_CUDA_CHECK(cudaGetLastError());
     }
   };
-  if ((M + LargeTile::BM - 1) / LargeTile::BM * cols * nz <= PVFMM_GEMM_SMALL)
+  if ((M + LargeTile::BM - 1) / LargeTile::BM * cols * nz <= kSmallTileBlocks)
     run(translate_gemm_kernel<SmallTile, Mode>, SmallTile::BM, SmallTile::smem);
   else
     run(translate_gemm_kernel<LargeTile, Mode>, LargeTile::BM, LargeTile::smem);
