@@ -18,6 +18,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <map>
 
 #include "fmm_context.cuh"
 
@@ -1213,12 +1215,111 @@ void build_tree(Context& ctx, const void* src_pos, long n_src, const void* trg_p
 
 }  // namespace pvfmm_b200
 
+// Runs link_nodes on the internal nodes of `levels` (sorted keys per level) in
+// arrays followed by guard bands and compares every array, guards included,
+// with links found by searching all node keys on the host.  A node whose
+// parent is missing is expected at the root, and reported.
+static void check_link_nodes(const std::vector<std::vector<pvfmm_b200::MKey>>& levels) {
+  using namespace pvfmm_b200;
+  constexpr long kGuard = 64;
+  LevelTab lt{};
+  lt.depth = (int)levels.size();
+  long n_int = 0, N = 1;
+  for (int d = 0; d < lt.depth; ++d) {
+    lt.n[d] = (long)levels[d].size();
+    lt.ioff[d] = n_int;
+    lt.off[d + 1] = N;
+    n_int += lt.n[d];
+    N += 8 * lt.n[d];
+  }
+  lt.off[lt.depth + 1] = N;
+  // expected arrays (guards: bytes 0x5a)
+  const int g4 = 0x5a5a5a5a;
+  std::vector<MKey> keys(N + kGuard, MKey{0x5a5a5a5a5a5a5a5aULL, 0x5a5a5a5au, 0x5a5a5a5au});
+  std::vector<unsigned char> leaf(N + kGuard, 0x5a);
+  std::vector<int> child0(N + kGuard, g4), parent(N + kGuard, g4), int_idx(n_int + kGuard, g4);
+  std::map<std::pair<unsigned long long, unsigned int>, long> where;  // node of a key
+  for (long i = 0; i < N; ++i) {
+    leaf[i] = 1;
+    child0[i] = -1;
+    parent[i] = 0;
+  }
+  keys[0] = make_key(0, 0, 0, 0);
+  parent[0] = -1;
+  where[{keys[0].hi, keys[0].lo}] = 0;
+  bool bad = false;
+  for (int d = 0; d < lt.depth; ++d)
+    for (long k = 0; k < lt.n[d]; ++k) {
+      const MKey& key = levels[d][k];
+      const auto it = where.find({key.hi, key.lo});
+      const long g = it == where.end() ? 0 : it->second;
+      bad = bad || it == where.end();
+      leaf[g] = 0;
+      child0[g] = (int)(lt.off[d + 1] + 8 * k);
+      int_idx[lt.ioff[d] + k] = (int)g;
+      unsigned int X, Y, Z, dd;
+      decode_key(key, X, Y, Z, dd);
+      const unsigned int w = kTwo30 >> (d + 1);
+      for (int c = 0; c < 8; ++c) {
+        const long i = lt.off[d + 1] + 8 * k + c;
+        keys[i] = make_key(X + (c & 1) * w, Y + (c >> 1 & 1) * w, Z + (c >> 2) * w, d + 1);
+        parent[i] = (int)g;
+        where[{keys[i].hi, keys[i].lo}] = i;
+      }
+    }
+  DevBuf b[7];
+  try {
+    MKey* S = b[0].as<MKey>(n_int);
+    MKey* dk = b[1].as<MKey>(keys.size());
+    unsigned char* dl = b[2].as<unsigned char>(leaf.size());
+    int* dc = b[3].as<int>(child0.size());
+    int* dp = b[4].as<int>(parent.size());
+    int* di = b[5].as<int>(int_idx.size());
+    int* db = b[6].as<int>(1);
+    for (int d = 0; d < lt.depth; ++d) {
+      lt.S[d] = S + lt.ioff[d];
+      PVFMM_CUDA_CHECK(cudaMemcpy(S + lt.ioff[d], levels[d].data(), lt.n[d] * sizeof(MKey), cudaMemcpyHostToDevice));
+    }
+    PVFMM_CUDA_CHECK(cudaMemset(dk, 0x5a, keys.size() * sizeof(MKey)));
+    PVFMM_CUDA_CHECK(cudaMemset(dl, 0x5a, leaf.size()));
+    PVFMM_CUDA_CHECK(cudaMemset(dl, 1, N));
+    PVFMM_CUDA_CHECK(cudaMemset(dc, 0x5a, child0.size() * sizeof(int)));
+    PVFMM_CUDA_CHECK(cudaMemset(dc, 0xff, N * sizeof(int)));
+    PVFMM_CUDA_CHECK(cudaMemset(dp, 0x5a, parent.size() * sizeof(int)));
+    PVFMM_CUDA_CHECK(cudaMemset(dp, 0, N * sizeof(int)));
+    PVFMM_CUDA_CHECK(cudaMemset(di, 0x5a, int_idx.size() * sizeof(int)));
+    PVFMM_CUDA_CHECK(cudaMemset(db, 0, sizeof(int)));
+    link_nodes<<<ceil_div(n_int, 128), 128>>>(lt, n_int, dk, dl, dc, dp, di, db);
+    PVFMM_CUDA_CHECK(cudaGetLastError());
+    auto same = [](const auto& want, const auto* dev, const char* name, size_t from) {
+      auto got = want;
+      const size_t es = sizeof(want[0]);
+      PVFMM_CUDA_CHECK(cudaMemcpy(got.data(), dev, want.size() * es, cudaMemcpyDeviceToHost));
+      for (size_t i = from; i < want.size(); ++i)
+        if (std::memcmp(&got[i], &want[i], es) != 0)
+          throw std::runtime_error(std::string("link_nodes: entry ") + std::to_string(i) + " of " + name);
+    };
+    same(std::vector<int>{bad}, db, "the error word", 0);
+    same(keys, dk, "keys", 0);
+    same(leaf, dl, "leaf", 0);
+    same(child0, dc, "child0", bad ? 1 : 0);  // (nodes without a parent share the root's entry)
+    same(parent, dp, "parent", 0);
+    same(int_idx, di, "int_idx", 0);
+  } catch (...) {
+    for (DevBuf& d : b) d.release();
+    throw;
+  }
+  for (DevBuf& d : b) d.release();
+}
+
 // Self-check of the bounded writes of the tree build (internal entry point,
 // used by the GPU tests; no counterpart in the reference).  Runs scatter_lists
 // with `n` nodes in every list against a capacity of `cap` < n, and link_nodes
-// on a set that is not closed, in buffers followed by a guard band, and checks
-// that what is in range is written and nothing beyond it.  Returns 0 when the
-// bounds hold, 1 otherwise (message in PVFMMGetLastError).
+// on a set that is not closed (n nodes of level 2 whose parents are missing)
+// and on closed ones of five levels (about n nodes), in buffers followed by
+// guard bands, and checks that what is in range is written as a host
+// computation has it and nothing beyond it.  Returns 0 when that holds, 1
+// otherwise (message in PVFMMGetLastError).
 extern "C" int PVFMMB200CheckBoundedWrites(long n, long cap) {
   using namespace pvfmm_b200;
   constexpr long kGuard = 64;
@@ -1263,46 +1364,23 @@ extern "C" int PVFMMB200CheckBoundedWrites(long n, long cap) {
         throw std::runtime_error("scatter_lists wrote the totals wrongly");
     cudaFree(buf);
     buf = nullptr;
-    // a root and, at level 2, n internal nodes whose parents are not in level
-    // 1 (one internal node, the last octant): 1 + 8 + 8 + 8 n tree nodes
-    const long N = 17 + 8 * n, NG = N + kGuard;
-    std::vector<MKey> S(n + 2);
-    S[0] = make_key(0, 0, 0, 0);
-    S[1] = make_key(kTwo30 / 2, kTwo30 / 2, kTwo30 / 2, 1);
-    for (long i = 0; i < n; ++i) S[2 + i] = make_key(0, 0, 0, 2);
-    const size_t bytes = (S.size() + NG) * sizeof(MKey) + (size_t)(2 * NG + n + 2 + kGuard + 1) * sizeof(int) + NG;
-    PVFMM_CUDA_CHECK(cudaMalloc(&buf, bytes));
-    PVFMM_CUDA_CHECK(cudaMemset(buf, 0, bytes));
-    MKey* dS = (MKey*)buf;
-    MKey* keys = dS + S.size();
-    int* child0 = (int*)(keys + NG);
-    int* parent = child0 + NG;
-    int* int_idx = parent + NG;
-    int* bad = int_idx + n + 2 + kGuard;
-    unsigned char* lf = (unsigned char*)(bad + 1);
-    PVFMM_CUDA_CHECK(cudaMemcpy(dS, S.data(), S.size() * sizeof(MKey), cudaMemcpyHostToDevice));
-    PVFMM_CUDA_CHECK(cudaMemset(child0, 0xff, 2 * NG * sizeof(int)));
-    LevelTab lt{};
-    lt.depth = 3;
-    const long cnts[3] = {1, 1, n};
-    lt.off[1] = 1;
-    for (int d = 0; d < 3; ++d) {
-      lt.S[d] = dS + lt.ioff[d];
-      lt.n[d] = cnts[d];
-      lt.ioff[d + 1] = lt.ioff[d] + cnts[d];
-      lt.off[d + 2 > 3 ? 3 : d + 1] = d == 0 ? 1 : d == 1 ? 9 : 17;
+    const MKey root = make_key(0, 0, 0, 0), far = make_key(kTwo30 / 2, kTwo30 / 2, kTwo30 / 2, 1);
+    check_link_nodes({{root}, {far}, std::vector<MKey>(n, make_key(0, 0, 0, 2))});
+    // closed sets: of each level's children every third, and the last two
+    std::vector<std::vector<MKey>> levels{{root}};
+    while (levels.size() < 5) {
+      const unsigned int d = (unsigned int)levels.size(), w = kTwo30 >> d;
+      std::vector<MKey> next;
+      long i = 0;
+      for (const MKey& key : levels.back()) {
+        unsigned int X, Y, Z, dd;
+        decode_key(key, X, Y, Z, dd);
+        for (unsigned int c = 0; c < 8 && (long)next.size() < n; ++c, ++i)
+          if (i % 3 == 0 || c >= 6) next.push_back(make_key(X + (c & 1) * w, Y + (c >> 1 & 1) * w, Z + (c >> 2) * w, d));
+      }
+      levels.push_back(next);
+      check_link_nodes(levels);
     }
-    lt.off[3] = 17;
-    link_nodes<<<ceil_div(n + 2, 128), 128>>>(lt, n + 2, keys, lf, child0, parent, int_idx, bad);
-    PVFMM_CUDA_CHECK(cudaGetLastError());
-    std::vector<int> hc(2 * NG);
-    int hb = 0;
-    PVFMM_CUDA_CHECK(cudaMemcpy(hc.data(), child0, 2 * NG * sizeof(int), cudaMemcpyDeviceToHost));
-    PVFMM_CUDA_CHECK(cudaMemcpy(&hb, bad, sizeof(int), cudaMemcpyDeviceToHost));
-    if (hb != 1) throw std::runtime_error("link_nodes did not report the missing parents");
-    for (long k = N; k < NG; ++k)
-      if (hc[k] != -1 || hc[NG + k] != -1) throw std::runtime_error("link_nodes wrote out of range");
-    cudaFree(buf);
     set_last_error("");
     return 0;
   } catch (const std::exception& e) {

@@ -357,16 +357,17 @@ def test_vlist_chunks_give_identical_results(monkeypatch, prec):
 
 
 def test_tree_build_writes_stay_in_bounds_on_a_count_mismatch():
-    """The tree build checks its per-level internal-node and leaf counts only
-    at its final synchronisation; until then the kernels that write by scan
-    rank skip ranks beyond the buffers' capacities.  The library's self-check
-    runs them with more flagged entries than capacity and checks a guard band
-    after each buffer."""
+    """The tree build learns that its counts do not fit, or that a node's
+    parent is missing, when the list totals are read back; until then its
+    kernels skip list ranks beyond the capacity and link such nodes to the
+    root.  The library's self-check runs them in both situations and on closed
+    trees, and compares every array and the guard band behind it with a host
+    computation."""
     lib = P.load_library()
     f = lib.PVFMMB200CheckBoundedWrites
     f.restype = ctypes.c_int
     f.argtypes = [ctypes.c_long, ctypes.c_long]
-    for n, cap in [(1000, 600), (4096, 0), (300, 300)]:
+    for n, cap in [(1000, 600), (4096, 0), (300, 300), (1, 1)]:
         assert f(n, cap) == 0, P.last_error()
 
 
@@ -375,8 +376,8 @@ def test_tcgen05_hadamard_agrees_with_mma_sync_hadamard(monkeypatch):
     (tcgen05, TMEM accumulators, tiles of Morton-consecutive targets with their
     source unions staged in shared memory) and on the warp-level MMA path give
     the same FMM result to well within the mixed form's accuracy (both carry
-    each product to ~2^-22 with a 3-term TF32 split; only the accumulation
-    order inside the tensor cores differs)."""
+    each product to ~2^-22 with a 3-term split, of TF32 and of FP16 halves; the
+    accumulation order inside the tensor cores differs too)."""
     src = points("gauss", 40000, 41)
     den = np.random.default_rng(42).uniform(-1, 1, 40000)
     monkeypatch.setenv("PVFMM_B200_HADAMARD", "tcgen05")
@@ -413,7 +414,7 @@ def test_fp64_tensor_core_hadamard_agrees_with_simt(monkeypatch, kid):
 @pytest.mark.parametrize("kid", [3, 2, 4, 5])
 def test_tensor_core_hadamard_of_vector_expansions_agrees_with_simt(monkeypatch, kid, prec):
     """The V-list products of the 3-component expansions (Stokes velocity,
-    pressure, velocity gradient; Biot-Savart) on the tensor cores (mixed: TF32
+    pressure, velocity gradient; Biot-Savart) on the tensor cores (mixed: FP16
     3-term split, plain: FP64; K = 48, streamed operator fragments) and in SIMT
     give the same FMM result: to FP64 rounding in the plain form (2e-13 apart:
     624-term sums in different orders, amplified by the downward
@@ -483,3 +484,20 @@ def test_double_layer_setup0_and_rejections():
     with pytest.raises(RuntimeError, match="double-layer"):
         g.evaluate(s, sl, dl1, t, True)
     g.close()
+
+
+def test_fp64_reciprocal_square_root():
+    """One source and one target a distance r apart: f / (4 pi r).  The FP64
+    kernels' 1/r is at most 1.4e-16 off over the whole range of r^2, subnormal
+    r^2 included; the product and the factor 1 / (4 pi) round once each (1.11e-16).
+    r has at most 26 significant bits, so that r^2 is exact."""
+    rng = np.random.default_rng(3)
+    exps = np.repeat(np.arange(-510, 511, 2), 200)
+    r = np.ldexp(rng.integers(1 << 25, 1 << 26, len(exps)).astype(float), exps - 26)
+    r = np.concatenate([r, np.ldexp(1.0, np.arange(-537, -510))])
+    trg = np.zeros((len(r), 3))
+    trg[np.arange(len(r)), rng.integers(0, 3, len(r))] = r * rng.choice([-1.0, 1.0], len(r))
+    out = P.kernel_eval(P.FMMKernel.LaplacePotential, np.zeros(3), np.ones(1), trg.reshape(-1))
+    pi = np.longdouble("3.14159265358979323846264338327950288")
+    want = 1 / (4 * pi * r.astype(np.longdouble))
+    assert float(np.max(np.abs(out.astype(np.longdouble) / want - 1))) < 1.4e-16 + 2 * 1.11e-16

@@ -89,13 +89,11 @@ def test_empty_parents_and_partial_tiles(monkeypatch, kernel, m, n):
     rng = np.random.default_rng(n)
     pos = rng.random((n, 3))
     q = rng.standard_normal((n, P.KERNEL_DIMS[kernel][0]))
-    q[pos[:, 0] < 0.5] = 0.0                        # parents whose spectra are all zero
-    q[pos[:, 0] > 0.9] *= 2.0 ** 30                 # and parents of a very different scale
-    x = pos.reshape(-1)
-    a = _ctx(kernel, m).evaluate(x, q.reshape(-1), None, x, True)
-    if P.KERNEL_DIMS[kernel][0] == 1:
-        b = _ctx(kernel, m, P.PRECISION_PLAIN).evaluate(x, q.reshape(-1), None, x, True)
-    else:
-        monkeypatch.setenv("PVFMM_B200_HADAMARD3", "simt")
-        b = _ctx(kernel, m).evaluate(x, q.reshape(-1), None, x, True)
+    # neighbouring parents with exponents of their own: 2^-6 .. 2^6 per cell of
+    # side 1/8, so that a parent left out or scaled by another's exponent costs
+    # 1e-4 of the result and more
+    cell = (pos * 8).astype(int)
+    q *= 2.0 ** rng.integers(-6, 7, 512)[cell[:, 0] * 64 + cell[:, 1] * 8 + cell[:, 2]][:, None]
+    q[pos[:, 0] < 0.25] = 0.0                       # parents whose spectra are all zero
+    a, b = _compare(monkeypatch, kernel, m, pos.reshape(-1), q.reshape(-1))
     assert _rel(a, b) < 1e-6
