@@ -102,7 +102,7 @@ __device__ inline long lower_bound_key(const MKey* a, long n, const MKey& k) {
 // FP64: the hardware estimate of rsqrt.approx.ftz.f64 (relative error at most
 // 9.3e-7, whole FP64 range) and one third-order step from the binomial series
 // of (1 - e)^(-1/2), e = 1 - r2 y^2: y <- y + y e (1/2 + 3/8 e), whose
-// remainder 5/16 e^3 is below 2^-59.  Measured over 2.7e8 arguments: at most
+// remainder 5/16 e^3 is at most 2.1e-18.  Measured over 2.7e8 arguments: at most
 // 1.4e-16 from 1/sqrt(r2).  Five FP64 operations and one special-function
 // one; two Newton steps from the FP32 estimate took seven, a double compare
 // and two FP64 <-> FP32 conversions (which run at half the special-function
@@ -128,7 +128,8 @@ __device__ __forceinline__ float rsqrt_nr(float r2) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(r2));
   const float y = y0 * (1.5f - 0.5f * r2 * y0 * y0);
   return r2 > 0.f ? y : 0.f;
-}// FP64 with one Newton step from the FP32 seed (relative error ~1e-13), for
+}
+// FP64 with one Newton step from the FP32 seed (relative error ~1e-13), for
 // r2 in the FP32 normal range; used where the pair distance is bounded away
 // from zero (equivalent-surface sources of the mixed form's D2T): one FP64
 // operation less than rsqrt_nr and no branch, which counts there (2M surface
