@@ -1,6 +1,8 @@
-"""V-list DFTs at the orders above 10 (one grid per block, long lines).
+"""V-list DFTs at the smallest order and at the large ones (few grids per block,
+long lines).
 
-Bars: the plain form against the direct sum, about four times the truncation
+Bars: the plain form against the oracle 1e-12 (the same operators, as in
+test_gpu_parity.py) and against the direct sum about four times the truncation
 error of these orders (2.7e-11 at m = 12, 1.2e-13 at m = 16, where FP64
 rounding takes over, with 200k uniform points); the mixed form's 1e-6.
 """
@@ -10,8 +12,21 @@ import numpy as np
 import pytest
 
 import pvfmm_b200 as P
+from oracle import pvfmm_oracle as O
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [2, 10, 12])
+def test_orders_match_oracle(m):
+    rng = np.random.default_rng(m)
+    x, q = rng.random((2000, 3)), rng.uniform(-1, 1, (2000, 1))
+    ops = O.Operators.from_arrays(O.KERNELS[0], m, P.precomp_operators(P.FMMKernel.LaplacePotential, m))
+    want = O.pvfmm_eval(0, m, 30, x, q, x, ops=ops)
+    ctx = P.FMMParticleContext(-1, 30, m, P.FMMKernel.LaplacePotential)
+    out = ctx.evaluate(x.reshape(-1), q.reshape(-1), None, x.reshape(-1), True)
+    assert ctx.tree_stats()["n_vtrg"] > 16
+    assert O.rel_l2(out.reshape(-1, 1), want) < 1e-12
 
 
 @pytest.mark.parametrize("m,bar", [(12, 1e-10), (16, 1e-12)])
