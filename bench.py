@@ -447,11 +447,10 @@ def cpu_baseline(args):
 # a launch processes (traffic grows in proportion).  Units: n_vsrc + n_vtrg for
 # the Hadamard kernels, n_trg for the near field.
 TRAFFIC_1M = {
-    ("hadamard", 4): {"bytes": 844786176 + 671260416, "units": 4768 + 4767},     # hadamard_tc_kernel
-    # hadamard_rd_kernel<double> capture; hadamard_dmma1_kernel reads and writes the same spectra
-    ("hadamard", 8): {"bytes": 1470638080 + 1367394304, "units": 4768 + 4767},
-    ("near_field", 4): {"bytes": 149489664 + 25314816, "units": 1000000},        # near_field_kernel<float>
-    ("near_field", 8): {"bytes": 151890688 + 20192256, "units": 1000000},        # near_field_kernel<double>
+    ("hadamard", 4): {"bytes": 802614016 + 667337472, "units": 4768 + 4767},     # hadamard_tc_kernel
+    ("hadamard", 8): {"bytes": 1569977088 + 1370500352, "units": 4768 + 4767},   # hadamard_dmma1_kernel
+    ("near_field", 4): {"bytes": 151397632 + 21148928, "units": 1000000},        # near_field_kernel<float>
+    ("near_field", 8): {"bytes": 151598592 + 20681984, "units": 1000000},        # near_field_kernel<double>
 }
 # kernel that computes the V-list Hadamard products: (real bytes, ke) -> name
 HADAMARD_KERNEL = {(4, 1): "hadamard_tc_kernel (V-list M2L, FP16 mma.sync x3 split)",

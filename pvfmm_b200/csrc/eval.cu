@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(kNF, sizeof(Real) == 8       ? PVFMM_NEAR_MIN_
 // one thread per pair would not fill the chip (surface_lanes).
 // Against one block per node with the sources in shared memory and two Newton
 // steps: 4M clustered points S2U with its products 3.15 -> 2.81 ms, X list
-// 0.48 -> 0.36 ms.
+// 0.48 -> 0.33 ms.
 // ---------------------------------------------------------------------------
 inline int surface_lanes(long n_pairs) { return n_pairs < 148L * 1024 ? 4 : 1; }
 
@@ -824,7 +824,14 @@ __global__ void __launch_bounds__(kNT) surface_check_kernel(
 // stored as hi = fp16(v 2^-E), lo = fp16(v 2^-E - hi) (22 bits and lo's sign,
 // as a TF32 hi/lo pair), with one exponent E per parent such that no value of
 // its spectra exceeds 2^15.  Values down to 2^-18 of that bound keep all 22
-// bits; below that the error stays at 2^-25, 2^-40 of the bound.
+// bits; below that the error stays at 2^-25, 2^-40 of the bound.  TF32 halves
+// kept 22 bits at any size, so a child much weaker than its strongest sibling
+// loses bits here; that sibling's own FP32 rounding (2^-24 of it) is larger
+// wherever its field reaches, which is everywhere the weak one's does.
+// Rms errors of potentials against the plain form, 100k points, 24 sets each,
+// over those of the TF32 form (and its plain DFT sums): m = 8 0.85 to 0.88,
+// m = 10 0.99 to 1.00; with densities times 2^0 .. 2^40 per cell of side 1/16
+// 0.86 to 0.87 and 0.97 to 1.01.
 // ---------------------------------------------------------------------------
 // (re, im) as two packed halves: their hi parts and their lo parts.
 __device__ __forceinline__ void half_split(float re, float im, unsigned& hi, unsigned& lo) {
@@ -1059,8 +1066,8 @@ struct FftSizes {
 // plain sums in the FP32 inverse, see idft_plain).
 // Against plain sums with the twiddles in shared memory, piece-major FP64
 // spectra and 4-byte FP16 stores, 4M clustered points in the mixed form:
-// forward 1.73 -> 0.99 ms, inverse 1.62 -> 1.37 ms; 1M in FP64: 1.89 -> 0.64
-// and 0.95 -> 0.56 ms.  What bounds the forward one now is its 64-byte row
+// forward 1.73 -> 1.00 ms, inverse 1.62 -> 1.37 ms; 1M in FP64: 1.98 -> 0.64
+// and 0.95 -> 0.67 ms.  What bounds the forward one now is its 64-byte row
 // stores at the frequency-major stride.
 // Output layout: frequency-major rows (split_row) for the scalar FP64
 // Hadamards, spec[f][q][child], and for the split-FP16 ones (`qinv` given),
@@ -1604,9 +1611,10 @@ __global__ void __launch_bounds__(128, 4) hadamard_rd_kernel(int n3h, long n_vtr
 // per 16 rows and offset).  Measured against that TF32 form: 4M clustered
 // points (m = 8, 16,037 parents) 10.8 -> 7.05 ms, 2M surface points 13.1 ->
 // 7.5 ms, 1M Stokes points (m = 6) 9.5 -> 6.1 ms; outputs 3e-9 to 9e-7 apart.
-// What bounds the scalar kernel now is the L1 data path (72% of its rate: 12
-// wavefronts for the two gathers of a tile and offset, 8 for the operator
-// fragments, 4 for scales and indices, against 13 cycles of MMA), with 59% of
+// What bounds the scalar kernel is the L1 data path (83% of its rate at 1M
+// clustered points, tensor pipe 34%, issue slots 59%: 12 wavefronts for the
+// two gathers of a tile and offset, 8 for the operator fragments, 4 for scales
+// and indices, against 13 cycles of MMA), with 49% of
 // the gathered sectors hit in L1; so the kernel keeps its shared memory small:
 // operator fragments 27 KB per block, 3 blocks per SM (4 blocks, with a
 // smaller L1, took 9.0 ms; two tiles per warp 7.7 ms).  Each warp prefetches
